@@ -1,0 +1,103 @@
+"""The chunked stage kernels on grids whose rows are not whole 16-byte units
+and on fields at unaligned addresses (linesolve_any.cu), against the CPU
+oracle with the bars of test_gpu_ops.py: tiles with a partial last column or
+row, lines one point around a multiple of the chunk (16 points FP64, 32
+FP32), an odd number of chunks, lines that need more than 256 threads a
+tile, and lines that leave only the 8-line tiles."""
+import numpy as np
+import pytest
+
+from conftest import rel_err, seeded_field
+from test_gpu_ops import ROUTINES, X, Y, Z, call
+
+pytestmark = pytest.mark.gpu
+
+LEN = (2 * np.pi, 1.5, 3.0)
+
+
+def _all_routines(oracle, ctx, u_d, make_out, shape, prec):
+    from x3div_b200 import to_host
+    used = to_host(u_d).astype(np.float64)
+    d = {X: ctx.dx, Y: ctx.dy, Z: ctx.dz}
+    tol = 1e-12 if prec == "f64" else 1e-5
+    for routine, opname, kind, direction, style in ROUTINES:
+        t_d = make_out()
+        call(ctx, routine, style, t_d, u_d, ctx.op(opname), shape)
+        ctx.sync()
+        assert ctx.last_kernel() in (0, 3), (routine, ctx.last_kernel())
+        err = rel_err(to_host(t_d), oracle.apply(kind, direction, used, d[direction]))
+        assert err < tol, (routine, opname, shape, prec, err)
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(17, 33, 31), (33, 16, 65), (49, 97, 32), (15, 300, 10), (271, 9, 12),
+                                   (9, 12, 1000), (1001, 8, 9)])
+def test_routines_on_odd_extents(oracle, torch_cuda, shape, prec):
+    torch = torch_cuda
+    from x3div_b200 import Context, to_device
+    ctx = Context(*shape, lengths=LEN, precision=prec)
+    u_d = to_device(seeded_field(shape, seed=sum(shape), noise=1e-2), torch.float64 if prec == "f64" else torch.float32)
+    _all_routines(oracle, ctx, u_d, lambda: torch.full_like(u_d, float("nan")), shape, prec)
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_routines_on_unaligned_fields(oracle, torch_cuda, prec):
+    """Input and output one element into their allocations."""
+    torch = torch_cuda
+    from x3div_b200 import Context, to_device
+    shape = (32, 24, 40)
+    ctx = Context(*shape, lengths=LEN, precision=prec)
+    u = to_device(seeded_field(shape, seed=5, noise=1e-2), torch.float64 if prec == "f64" else torch.float32)
+
+    def shifted():
+        return torch.full((u.numel() + 1,), float("nan"), dtype=u.dtype, device="cuda")[1:].view(u.shape)
+
+    u_d = shifted()
+    u_d.copy_(u)
+    _all_routines(oracle, ctx, u_d, shifted, shape, prec)
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(17, 12, 10), (34, 33, 18), (45, 16, 33), (9, 290, 12)])
+def test_stages_on_odd_extents(oracle, torch_cuda, shape, prec):
+    """divergence, gradp, momentum_rhs_eq and an Euler step in three fused
+    launches a stage, with the bars of test_gpu_stages.py (FP32: an
+    interpolation alone is about 6e-6 and a stage chains three operators)."""
+    torch = torch_cuda
+    from x3div_b200 import Context, to_device, to_host
+    ctx = Context(*shape, lengths=LEN, precision=prec)
+    dt_ = torch.float64 if prec == "f64" else torch.float32
+    tol = 1e-12 if prec == "f64" else 1e-4
+    u = [to_device(seeded_field(shape, s, lengths=LEN, noise=1e-2), dt_) for s in (1, 2, 3)]
+    uh = [to_host(a).astype(np.float64) for a in u]
+    h = (ctx.dx, ctx.dy, ctx.dz)
+    p = torch.empty(shape[::-1], dtype=torch.float64, device="cuda")
+    n0 = ctx.launch_count()
+    ctx.divergence(p, *u)
+    assert ctx.launch_count() - n0 == 3
+    assert rel_err(to_host(p), oracle.divergence(*uh, *h)) < tol
+    ph = seeded_field(shape, 30, kind="rand", lengths=LEN, noise=0)
+    pd = to_device(ph)
+    g, du = ([torch.empty_like(u[0]) for _ in range(3)] for _ in range(2))
+    ctx.gradp(*g, pd)
+    assert ctx.launch_count() - n0 == 6
+    ctx.momentum_rhs_eq(*du, *u)
+    assert ctx.launch_count() - n0 == 9
+    ctx.sync()
+    for got, want in zip(g, oracle.gradp(ph, *h)):
+        assert rel_err(to_host(got), want) < tol
+    for got, want in zip(du, oracle.momentum_rhs(*uh, *h)):
+        assert rel_err(to_host(got), want) < tol
+    ctx.euler_step(*u, *du, p, *g, 1e-3)
+    ctx.sync()
+    oracle.euler_step(*uh, 1e-3, lengths=LEN)
+    # the divergence carries the unit roundoff times the interpolation's
+    # condition (99) times the largest wavenumber (2 / h), and the projection
+    # divides it by the smallest one (2 pi / L): on (9, 290, 12) the cells are
+    # a hundred times flatter than long, and FP32 gives 2.3e-3
+    bound = 99 * 2 / min(h) * max(LEN) / (2 * np.pi) * (2.0**-53 if prec == "f64" else 2.0**-24)
+    for got, want in zip(u, uh):
+        assert rel_err(to_host(got), want) < max(bound, 1e-11 if prec == "f64" else 1e-4)
+    ctx.close()

@@ -55,6 +55,7 @@ struct StageProgram {
     int nops, ntiles;
     int prefetch_mask;  // bit k: operator k's base is prefetched (set by launch_stage)
     int in_f64;         // T = float: in[] hold FP64 fields (y/z plain programs only)
+    int aligned_only;   // refuse extents and addresses that need linesolve_any.cu
 };
 
 // Number of (lines per CTA, chunk length, persistence, lines per thread)
@@ -73,6 +74,12 @@ inline bool is_stage_cfg(int cfg) { return cfg >= 0 && cfg < kAllConfigs && cfg 
 template <typename T>
 int launch_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, int nx, int ny, int nz,
                  int cfg);
+
+// The same program on a grid whose rows or addresses are not whole 16-byte
+// units, W lines per CTA in chunks of kChunkLong<T> points (linesolve_any.cu);
+// launch_stage's configurations 0 (W = 16) and 3 (W = 8) fall through to it.
+template <typename T, int W>
+int launch_stage_any(x3d_ctx_s *ctx, const StageProgram<T> &prog, bool acc, int dir, int nx, int ny, int nz);
 
 // One job of a box batch: up to six operators applied along one direction to
 // one field of one box.  Filled on the host, read by the persistent batch

@@ -128,6 +128,17 @@ __device__ __forceinline__ void bulk_wait_read_all()
 // Wait until every committed bulk group of this thread has completed.
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
+// Asynchronous copy of one 4- or 8-byte element global -> shared memory (any
+// element-aligned address), and the wait for all of this thread's.
+template <int BYTES>
+__device__ __forceinline__ void cp_async(void *dst, const void *src)
+{
+    static_assert(BYTES == 4 || BYTES == 8, "one element");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Make generic-proxy writes to shared memory visible to the async proxy.
 __device__ __forceinline__ void fence_proxy_async_smem()
 {

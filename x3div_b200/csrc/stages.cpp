@@ -62,9 +62,12 @@ static void set_flush(StageOp<T> &s, void *out, const void *base = nullptr, bool
 }
 
 // Local extents of the field a stage runs on: the context's box, or a
-// pencil of it whose lines along the stage's direction are whole.
+// pencil of it whose lines along the stage's direction are whole.  aligned_only:
+// the caller composes the stage from other kernels, or refuses it, where rows
+// are not whole 16-byte units (the pencil parts and x3d_divergence_noalloc).
 struct Ext {
     int nx, ny, nz;
+    bool aligned_only = false;
 };
 
 static Ext box_ext(const x3d_ctx_s *ctx) { return {ctx->nx, ctx->ny, ctx->nz}; }
@@ -138,10 +141,12 @@ static int run_program(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, con
 // launch per part of split_by_inputs (stages "<name>.1", "<name>.2", ...).
 // While tuning, times both forms and records the choice as "<name>.parts".
 template <typename T>
-static int run_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, const char *cname, Ext e)
+static int run_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int dir, const char *cname, Ext e)
 {
     const TraceRange trace(cname);
     const std::string name = stage_key(ctx, cname, e);
+    StageProgram<T> prog = prog_in;
+    prog.aligned_only = e.aligned_only;
     StageProgram<T> part[kMaxStageOps];
     const int nparts = split_by_inputs<T>(prog, part);
     const auto it = ctx->stage_tuned.find(name + ".parts");
@@ -304,9 +309,11 @@ static int divergence_dir(x3d_ctx_s *ctx, int dir, void *const *out, const void 
 }
 
 template <typename T>
-static int divergence_t(x3d_ctx_s *ctx, double *pp3, const void *const u[3], void *const s[5])
+static int divergence_t(x3d_ctx_s *ctx, double *pp3, const void *const u[3], void *const s[5],
+                        bool aligned_only = false)
 {
-    const Ext e = box_ext(ctx);
+    Ext e = box_ext(ctx);
+    e.aligned_only = aligned_only;
     int rc = divergence_dir<T>(ctx, DX, s, u, e);
     void *const y_out[2] = {s[3], s[4]};
     const void *const y_in[3] = {s[0], s[1], s[2]};
@@ -409,10 +416,12 @@ int fused_divergence(x3d_ctx_s *ctx, double *pp3, const void *const u[3])
 }
 
 // The fused divergence on caller-provided intermediate fields s[0..4] (each
-// nx*ny*nz elements of the context precision); allocates nothing.
+// nx*ny*nz elements of the context precision); allocates nothing, and takes
+// only grids whose rows are whole 16-byte units.
 int fused_divergence_scratch(x3d_ctx_s *ctx, double *pp3, const void *const u[3], void *const s[5])
 {
-    return ctx->precision == X3D_F32 ? divergence_t<float>(ctx, pp3, u, s) : divergence_t<double>(ctx, pp3, u, s);
+    return ctx->precision == X3D_F32 ? divergence_t<float>(ctx, pp3, u, s, true)
+                                     : divergence_t<double>(ctx, pp3, u, s, true);
 }
 
 int fused_gradp(x3d_ctx_s *ctx, void *const px[3], const double *pp3, void *const ucor[3])
@@ -428,14 +437,14 @@ int fused_gradp(x3d_ctx_s *ctx, void *const px[3], const double *pp3, void *cons
 int part_transeq(x3d_ctx_s *ctx, int dir, void *const du[3], const void *const u[3], const void *const *add,
                  void *const *unew, double dt, int nx, int ny, int nz)
 {
-    const Ext e{nx, ny, nz};
+    const Ext e{nx, ny, nz, true};
     return ctx->precision == X3D_F32 ? transeq_dir<float>(ctx, dir, du, u, add, unew, dt, e)
                                      : transeq_dir<double>(ctx, dir, du, u, add, unew, dt, e);
 }
 
 int part_divergence(x3d_ctx_s *ctx, int dir, void *const *out, const void *const *in, int nx, int ny, int nz)
 {
-    const Ext e{nx, ny, nz};
+    const Ext e{nx, ny, nz, true};
     return ctx->precision == X3D_F32 ? divergence_dir<float>(ctx, dir, out, in, e)
                                      : divergence_dir<double>(ctx, dir, out, in, e);
 }
@@ -443,7 +452,7 @@ int part_divergence(x3d_ctx_s *ctx, int dir, void *const *out, const void *const
 int part_gradp(x3d_ctx_s *ctx, int dir, void *const *out, const void *const *in, void *const *ucor, int nx, int ny,
                int nz)
 {
-    const Ext e{nx, ny, nz};
+    const Ext e{nx, ny, nz, true};
     return ctx->precision == X3D_F32 ? gradp_dir<float>(ctx, dir, out, in, ucor, e, nullptr)
                                      : gradp_dir<double>(ctx, dir, out, in, ucor, e, nullptr);
 }
