@@ -316,6 +316,52 @@ void finish_op(OpHost &op)
         op.den = 1.0;
 }
 
+// The tables of a non-periodic operator's chunked solve for chunks of L points
+// (see linesolve_walls.cu): rows of C L entries s, w, fw, H, G, then the
+// chunks' forward and backward multipliers.  With P_i the product of -s from
+// the chunk's start to i, H_i = w_i P_i - fw_i H_{i+1} and G_i the product of
+// -fw from i to the chunk's end.  Entries past the line's end are zero.
+// Returns the scan depth for thr, or -1 where a factor is not finite or a
+// multiplier above 1 would let a carry grow (no operator of the library).
+static int build_wall_tables(const OpHost &h, int L, double thr, std::vector<double> &tab)
+{
+    const int n = h.n, C = (n + L - 1) / L, P = C * L;
+    tab.assign((size_t)5 * P + 2 * C, 0.0);
+    double *s = tab.data(), *w = s + P, *fw = w + P, *H = fw + P, *G = H + P, *mf = G + P, *mb = mf + C;
+    for (int i = 0; i < n; ++i) {
+        s[i] = h.s[i];
+        w[i] = h.w[i];
+        fw[i] = h.f[i] * h.w[i];
+    }
+    for (int c = 0; c < C; ++c) {
+        const int b = c * L, e = std::min(n, b + L);
+        std::vector<double> p(e - b);
+        double q = 1.0;
+        for (int i = b; i < e; ++i) p[i - b] = (q *= -s[i]);
+        mf[c] = q;
+        double hn = 0.0, g = 1.0;
+        for (int i = e - 1; i >= b; --i) {
+            H[i] = hn = w[i] * p[i - b] - fw[i] * hn;
+            G[i] = g *= -fw[i];
+        }
+        mb[c] = g;
+    }
+    for (const double v : tab)
+        if (!std::isfinite(v)) return -1;
+    int depth = 1;
+    // no chunk takes a carry from the last one forward or the first one backward
+    mf[C - 1] = mb[0] = 0.0;
+    for (const double *m : {mf, mb})
+        for (int c = 0; c < C; ++c) {
+            if (std::fabs(m[c]) > 1.0) return -1;
+            double prod = 1.0;
+            int k = 0;
+            for (; c + k < C && prod >= thr; ++k) prod *= std::fabs(m[c + k]);
+            depth = std::max(depth, k);
+        }
+    return depth;
+}
+
 // Scan depths for chunk length L: smallest k such that any k consecutive
 // chunk multipliers multiply to below 1e-20 (capped at the chunk count).
 int upload_op(x3d_op_s *op)
@@ -325,7 +371,17 @@ int upload_op(x3d_op_s *op)
     // layout (bytes, each part 256-aligned): float s,w,fw,p | double s,w,fw,p,g
     auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
     const size_t o_f = 0, o_d = al(o_f + 4 * n * sizeof(float));
-    const size_t total = al(o_d + 5 * n * sizeof(double));
+    // non-periodic operators: the chunked solve's tables, float then double
+    std::vector<double> wall[2];
+    bool walls = !h.periodic;
+    if (walls) {
+        op->wall_depth[0] = build_wall_tables(h, kChunkLong<float>, 1e-12, wall[0]);
+        op->wall_depth[1] = build_wall_tables(h, kChunkLong<double>, 1e-20, wall[1]);
+        walls = op->wall_depth[0] > 0 && op->wall_depth[1] > 0;
+    }
+    const size_t o_wf = al(o_d + 5 * n * sizeof(double));
+    const size_t o_wd = o_wf + (walls ? al(wall[0].size() * sizeof(float)) : 0);
+    const size_t total = o_wd + (walls ? al(wall[1].size() * sizeof(double)) : 0);
     std::vector<unsigned char> host(total, 0);
     float *hf = reinterpret_cast<float *>(host.data() + o_f);
     double *hd = reinterpret_cast<double *>(host.data() + o_d);
@@ -342,14 +398,24 @@ int upload_op(x3d_op_s *op)
         hd[3 * n + i] = p;
         hd[4 * n + i] = h.g[i];
     }
+    if (walls) {
+        std::copy(wall[0].begin(), wall[0].end(), reinterpret_cast<float *>(host.data() + o_wf));
+        std::copy(wall[1].begin(), wall[1].end(), reinterpret_cast<double *>(host.data() + o_wd));
+    }
     if (op->dmem) cudaFree(op->dmem);
     op->dmem = nullptr;
+    op->wallf = nullptr;
+    op->walld = nullptr;
     if (cudaMalloc(&op->dmem, host.size()) != cudaSuccess) return X3D_ENOMEM;
     if (cudaMemcpy(op->dmem, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess)
         return X3D_ECUDA;
     const unsigned char *base = static_cast<const unsigned char *>(op->dmem);
     const float *df = reinterpret_cast<const float *>(base + o_f);
     const double *dd = reinterpret_cast<const double *>(base + o_d);
+    if (walls) {
+        op->wallf = reinterpret_cast<const float *>(base + o_wf);
+        op->walld = reinterpret_cast<const double *>(base + o_wd);
+    }
     auto fill = [&](auto &lo, auto *arr) {
         lo.s = arr + 0 * n;
         lo.w = arr + 1 * n;

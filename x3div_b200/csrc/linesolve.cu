@@ -34,6 +34,7 @@
 #include <algorithm>
 #include <cstdio>
 
+#include "der_closure.cuh"
 #include "linesolve_chunk.h"
 #include "ptx.cuh"
 #include "x3d_internal.h"
@@ -62,37 +63,6 @@ __device__ __forceinline__ T stencil(const T *v, const LineOp<T> &op)
         return op.a * (v[4] + v[3]) + op.b * (v[5] + v[2]) + op.c * (v[6] + v[1]) + op.d * (v[7] + v[0]);
     if constexpr (KIND == IDENT) return v[4];
     return T(0);
-}
-
-// Right-hand side at the first two and last two points of a non-periodic
-// first-derivative line (der?_ij, src/x3d_derive.f90:171-210): v is the same
-// 9-point window (v[k] = u_{i-4+k}; entries past the line's ends are never
-// used here).  Free slip (ncl = 1) mirrors the field (npaire = 1: even, so
-// the derivative vanishes at the wall; npaire = 0: odd); Dirichlet (ncl = 2)
-// uses the one-sided closures.  Other points keep the interior stencil r.
-template <typename T>
-__device__ __forceinline__ T der_closure(int i, int n, const T *v, const LineOp<T> &op, T r)
-{
-    const T a = op.a, b = op.b;
-    if (i == 0) {
-        if (op.ncl1 == 1) return op.npaire == 1 ? T(0) : a * (v[5] + v[5]) + b * (v[6] + v[6]);
-        return op.cl[0] * v[4] + op.cl[1] * v[5] + op.cl[2] * v[6];
-    }
-    if (i == 1) {
-        if (op.ncl1 == 1)
-            return op.npaire == 1 ? a * (v[5] - v[3]) + b * (v[6] - v[4]) : a * (v[5] - v[3]) + b * (v[6] + v[4]);
-        return op.cl[3] * (v[5] - v[3]);
-    }
-    if (i == n - 2) {
-        if (op.ncln == 1)
-            return op.npaire == 1 ? a * (v[5] - v[3]) + b * (v[4] - v[2]) : a * (v[5] - v[3]) + b * ((-v[4]) - v[2]);
-        return op.cl[4] * (v[5] - v[3]);
-    }
-    if (i == n - 1) {
-        if (op.ncln == 1) return op.npaire == 1 ? T(0) : a * ((-v[3]) - v[3]) + b * ((-v[2]) - v[2]);
-        return -op.cl[5] * v[4] - op.cl[6] * v[3] - op.cl[7] * v[2];
-    }
-    return r;
 }
 
 template <typename T>
@@ -556,6 +526,18 @@ static int run_chunk(x3d_ctx_s *ctx, int dir, const void *in, const x3d_op_s *co
                      const int *kinds, void *const *outs, int nops, int nx, int ny, int nz, int cfg)
 {
     const LineOp<T> *lops[kMaxStageOps];
+    if (cfg == 0 && !ops[0]->h.periodic) {  // non-periodic operators: one chunked launch each
+        for (int k = 0; k < nops; ++k)
+            if (ops[k]->h.periodic || kinds[k] != DER || !ops[k]->wallf || outs[k] == in) return X3D_EUNSUPPORTED;
+        const int n_in = dir == DX ? nx : (dir == DY ? ny : nz);
+        for (int k = 0; k < nops; ++k) {
+            const int rc = launch_wall(ctx, ops[k], DER, dir, in, outs[k], n_in, dir == DX ? ny : nx,
+                                       dir == DZ ? ny : nz, kReflEven, sizeof(T) == 4);
+            if (rc) return rc;
+        }
+        ctx->last_cfg = cfg;
+        return X3D_OK;
+    }
     for (int k = 0; k < nops; ++k) {
         lops[k] = &lineop<T>(ops[k]);
         if (kinds[k] == IDENT || outs[k] == in) return X3D_EUNSUPPORTED;  // in-place Thomas: other paths
@@ -660,6 +642,8 @@ int launch_np_stag(x3d_ctx_s *ctx, const x3d_op_s *op, int dir, const void *in, 
         return set_error(ctx, X3D_EUNSUPPORTED,
                          "this staggered routine has a non-periodic branch for npaire 1 only (src/x3d_staggered.f90)");
     }
+    const int rc = launch_wall(ctx, op, kind, dir, in, out, n_in, o1, o2, refl, fp32);
+    if (rc != X3D_EUNSUPPORTED) return rc;
     const long nl = (long)o1 * o2;
     const int bs = 128;
     const unsigned grid = (unsigned)((nl + bs - 1) / bs);

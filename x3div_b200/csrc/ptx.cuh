@@ -128,13 +128,16 @@ __device__ __forceinline__ void bulk_wait_read_all()
 // Wait until every committed bulk group of this thread has completed.
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
-// Asynchronous copy of one 4- or 8-byte element global -> shared memory (any
-// element-aligned address), and the wait for all of this thread's.
+// Asynchronous copy of 4, 8 or 16 bytes global -> shared memory (both addresses
+// aligned to that size), and the wait for all of this thread's.
 template <int BYTES>
 __device__ __forceinline__ void cp_async(void *dst, const void *src)
 {
-    static_assert(BYTES == 4 || BYTES == 8, "one element");
-    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
+    static_assert(BYTES == 4 || BYTES == 8 || BYTES == 16, "a cp.async size");
+    if constexpr (BYTES == 16)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(dst)), "l"(src), "n"(BYTES) : "memory");
 }
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }

@@ -84,6 +84,12 @@ struct x3d_op_s {
     x3d::LineOp<float> opf{};
     x3d::LineOp<double> opd{};
     bool builtin = false;
+    // Non-periodic operators: the chunked solve's tables (linesolve_walls.cu),
+    // inside dmem; null where the factors do not bound the sweeps.  wall_depth:
+    // chunks a carry scan visits, FP32 and FP64.
+    const float *wallf = nullptr;
+    const double *walld = nullptr;
+    int wall_depth[2] = {0, 0};
 };
 
 struct x3d_ctx_s {
@@ -194,6 +200,10 @@ void free_op(x3d_op_s *op);
 // the (nx,ny,nz) field in -> out (may alias for kind IDENT).
 int launch_linesolve(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, const void *in,
                      void *out, int nx, int ny, int nz, bool fp32);
+// A non-periodic operator as a chunked solve (linesolve_walls.cu):
+// X3D_EUNSUPPORTED, launching nothing, when its lines do not fit.
+int launch_wall(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, const void *in, void *out, int n_in, int o1,
+                int o2, int refl, bool fp32);
 // Up to six operators along one direction applied to one input, one output each.
 int launch_group(x3d_ctx_s *ctx, int dir, const void *in, const x3d_op_s *const *ops,
                  const int *kinds, void *const *outs, int nops, int nx, int ny, int nz, bool fp32);
