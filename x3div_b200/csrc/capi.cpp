@@ -784,7 +784,7 @@ int x3d_ctx_set_kernel(x3d_ctx ctx, int cfg)
     ctx->tuned.clear();
     ctx->stage_tuned.clear();
     ctx->stage_ms.clear();
-    ctx->default_cfg = cfg < 0 ? 0 : cfg;
+    ctx->default_cfg = cfg < 0 ? -1 : cfg;
     return X3D_OK;
 }
 

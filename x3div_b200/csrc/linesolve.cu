@@ -568,11 +568,17 @@ int launch_group(x3d_ctx_s *ctx, int dir, const void *in, const x3d_op_s *const 
 {
     if (nops < 1 || nops > kMaxStageOps) return set_error(ctx, X3D_EINVAL, "bad operator group");
     const auto it = ctx->tuned.find(tune_key(dir, nx, ny, nz, fp32, nops));
-    const int first = it != ctx->tuned.end() ? it->second : ctx->default_cfg;
-    int rc = run_cfg(ctx, first, dir, in, ops, kinds, outs, nops, nx, ny, nz, fp32);
-    if (rc != X3D_EUNSUPPORTED) return rc;
+    DefaultCfgs pick{1, {0}};
+    if (it != ctx->tuned.end()) pick.cfg[0] = it->second;
+    else if (ctx->default_cfg >= 0) pick.cfg[0] = ctx->default_cfg;
+    else if (ops[0]->h.periodic)
+        pick = default_cfgs(fp32 ? 4 : 8, dir, ops[0]->h.n, (size_t)nx * ny * nz, 1, false, false);
+    int rc = X3D_EUNSUPPORTED;
+    for (int i = 0; i < pick.count; ++i) {
+        rc = run_cfg(ctx, pick.cfg[i], dir, in, ops, kinds, outs, nops, nx, ny, nz, fp32);
+        if (rc != X3D_EUNSUPPORTED) return rc;
+    }
     for (int cfg = 0; cfg < kAllConfigs; ++cfg) {
-        if (cfg == first) continue;
         rc = run_cfg(ctx, cfg, dir, in, ops, kinds, outs, nops, nx, ny, nz, fp32);
         if (rc != X3D_EUNSUPPORTED) return rc;
     }

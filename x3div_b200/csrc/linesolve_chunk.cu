@@ -619,16 +619,10 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_tiled()
     return fn;
 }
 
-struct StageOpView {
-    short flush, accumulate, mul_tile;
-};
-
 static size_t scratch_bytes(int C, int W, size_t es) { return ((size_t)2 * C * W * es + 15) & ~(size_t)15; }
 
 static bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 static bool al8(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 7) == 0; }
-
-static bool plain(const StageOpView &v) { return v.flush && !v.accumulate && v.mul_tile < 0; }
 
 template <typename Kern>
 static unsigned persistent_grid(x3d_ctx_s *ctx, Kern kern, int threads, size_t smem, long ntiles)
@@ -672,7 +666,6 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         return X3D_EUNSUPPORTED;
     } else {
         StageProgram<T> prog = prog_in;
-        fill_resp(prog, L, prog.ops[0].op.n);
         // base2 that is a staged input comes from shared memory; T-typed bases
         // are prefetched into L2 with the tile's inputs
         for (int k = 0; k < prog.nops; ++k) {
@@ -687,12 +680,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
             if (prog.ops[k].prefetch_base) prog.prefetch_mask |= 1 << k;
         // the ACC kernels carry the accumulator and every flush form; the
         // others only plain operators (out = the solve)
-        bool acc = false;
-        for (int k = 0; k < prog.nops; ++k) {
-            const StageOp<T> &so = prog.ops[k];
-            acc = acc || !plain(StageOpView{so.flush, so.accumulate, so.mul_tile}) ||
-                  (so.flush && (so.base || so.out2 || so.out_f64 || so.sign != 1.0));
-        }
+        const bool acc = program_acc(prog);
         const int n = prog.ops[0].op.n;
         for (int k = 0; k < prog.nops; ++k)
             if (!prog.ops[k].op.circ || prog.ops[k].op.n != n) return X3D_EUNSUPPORTED;
@@ -707,7 +695,10 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         const size_t resp_bytes = (size_t)prog.nops * 4 * L * es * PR;
         if (!whole_vectors(prog, dir, nx)) {
             if constexpr (PR == 1 && OCC == 1 && !PERSIST && L == kChunkLong<T> && W <= 16)
-                if (!prog.aligned_only) return launch_stage_any<T, W>(ctx, prog, acc, dir, nx, ny, nz);
+                if (!prog.aligned_only) {
+                    fill_resp(prog, L, n);
+                    return launch_stage_any<T, W>(ctx, prog, acc, dir, nx, ny, nz);
+                }
             return X3D_EUNSUPPORTED;
         }
         if (threads > kStageThreads<T, L, PR> || threads % 32) return X3D_EUNSUPPORTED;
@@ -732,6 +723,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                                  ~(size_t)127) +
                                 (size_t)W * pitch * es;
             if (smem + 1024 > ctx->smem_optin) return X3D_EUNSUPPORTED;
+            fill_resp(prog, L, n);
             auto kern = ls_stage_x<T, W, L, false, PERSIST, OCC>;
             if constexpr (OCC == 1)  // the OCC > 1 kernels take plain programs only
                 if (acc) kern = ls_stage_x<T, W, L, true, PERSIST>;
@@ -762,6 +754,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         const size_t tile = ((size_t)rows * W * esi + 127) & ~(size_t)127;
         const size_t smem = (PERSIST ? 2 : 1) * prog.ntiles * tile + scratch_bytes(C, W, es) + resp_bytes;
         if (smem + 1024 > ctx->smem_optin) return X3D_EUNSUPPORTED;
+        fill_resp(prog, L, n);
         StageMaps maps;
         std::memset(&maps, 0, sizeof(maps));
         auto encode = [&](CUtensorMap *m, const void *ptr, int rows_in_box, size_t eb) {
@@ -862,6 +855,55 @@ static int launch_stage_sel(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir
     case 20: return launch_stage_cfg<T, 16, Lbig, false, 1, 3>(ctx, prog, dir, nx, ny, nz);
     default: return X3D_EUNSUPPORTED;
     }
+}
+
+// Measured on cubes of 16 to 384 points a side, every configuration on the
+// operator groups (one and six operators) and on the nine fused stages of a
+// step.  The lines:
+//   fields up to 4 MiB (96^3 FP32, 64^3 FP64): the launch ends before every SM
+//     is busy, so the short chunk, whose serial sweeps are half as long, wins
+//     (64^3 FP32, six y operators: 8.6 us on configuration 4, 17.9 on 0;
+//     momentum y 10.9 against 20.4);
+//   up to 16 MiB (128^3): wider tiles or a pair of lines a thread in FP32 (six
+//     y operators 18.2 on 14, 21.2 on 0), one CTA per tile in FP64;
+//   above: the kernels built for three CTAs per SM for plain programs (384^3
+//     FP64, six y operators: 673 us on 19, 1051 on 0; 256^3 FP32 y 113 on 20,
+//     127 on 0), pairs for accumulating FP32 y/z programs (256^3 momentum z 198
+//     on 14, 236 on 0) and 8-line tiles for FP64 x ones, whose three staged
+//     fields then fit more CTAs (256^3 momentum x 313 on 3, 460 on 0).
+// The persistent configurations are left to the autotuner, although 17 is up
+// to 8 % ahead of 20: they claim tiles from the context's one counter, and an
+// untuned context may be moved between streams with launches in flight.
+DefaultCfgs default_cfgs(size_t es, int dir, int n, size_t points, int ntiles, bool acc, bool in64)
+{
+    const bool f32 = es == 4;
+    const size_t bytes = points * es;
+    const bool small = bytes <= (size_t)4 << 20, mid = bytes <= (size_t)16 << 20;
+    if (dir == DX) {
+        if (small) return {5, {2, 4, 5, 1, 0}};
+        if (acc) {
+            if (f32 && mid) return {3, {2, 5, 0}};
+            if (f32) return {2, {0, 3}};
+            return {3, {3, 1, 0}};
+        }
+        if (f32 && ntiles > 1) return {4, {5, 2, 19, 0}};
+        if (f32 && (mid || n < 256)) return {4, {20, 19, 0, 1}};
+        return {4, {19, 20, 3, 0}};
+    }
+    if (small) return {5, {4, 2, 1, 0, 5}};
+    if (acc) {
+        if (f32 && mid) return {3, {1, 14, 0}};
+        if (f32) return {3, {14, 1, 0}};
+        if (mid) return {3, {1, 0, 3}};
+        if (ntiles < 3 && n > 256) return {3, {3, 0, 1}};
+        return {3, {0, 3, 1}};
+    }
+    if (in64) {
+        if (mid) return {2, {1, 0}};
+        return {2, {0, 3}};
+    }
+    if (f32 && mid) return {4, {14, 1, 20, 0}};
+    return {3, {20, 19, 0}};
 }
 
 template <typename T>

@@ -75,6 +75,29 @@ template <typename T>
 int launch_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, int nx, int ny, int nz,
                  int cfg);
 
+// Up to kMaxDefaultCfgs configurations for a program that the autotuner has not
+// timed, best first, by the rule at default_cfgs (linesolve_chunk.cu).
+constexpr int kMaxDefaultCfgs = 5;
+struct DefaultCfgs {
+    int count, cfg[kMaxDefaultCfgs];
+};
+// es: element bytes of the context; n: points a line; points: of the field;
+// ntiles: staged inputs; acc: the program accumulates or flushes other than
+// plainly; in64: FP64 inputs of an FP32 program.
+DefaultCfgs default_cfgs(size_t es, int dir, int n, size_t points, int ntiles, bool acc, bool in64);
+
+// Whether a program needs the kernels with the accumulator and every flush form.
+template <typename T>
+inline bool program_acc(const StageProgram<T> &p)
+{
+    for (int k = 0; k < p.nops; ++k) {
+        const StageOp<T> &so = p.ops[k];
+        if (!so.flush || so.accumulate || so.mul_tile >= 0 || so.base || so.out2 || so.out_f64 || so.sign != 1.0)
+            return true;
+    }
+    return false;
+}
+
 // The same program on a grid whose rows or addresses are not whole 16-byte
 // units, W lines per CTA in chunks of kChunkLong<T> points (linesolve_any.cu);
 // launch_stage's configurations 0 (W = 16) and 3 (W = 8) fall through to it.

@@ -129,11 +129,17 @@ static int run_program(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, con
 {
     if (ctx->stage_tuning) return tune_stage<T>(ctx, prog, dir, name.c_str(), e);
     const auto it = ctx->stage_tuned.find(name);
-    const int first = it != ctx->stage_tuned.end() ? it->second
-                                                   : (is_stage_cfg(ctx->default_cfg) ? ctx->default_cfg : 0);
-    int rc = launch_stage<T>(ctx, prog, dir, e.nx, e.ny, e.nz, first);
+    DefaultCfgs pick{1, {0}};
+    if (it != ctx->stage_tuned.end()) pick.cfg[0] = it->second;
+    else if (is_stage_cfg(ctx->default_cfg)) pick.cfg[0] = ctx->default_cfg;
+    else
+        pick = default_cfgs(sizeof(T), dir, prog.ops[0].op.n, (size_t)e.nx * e.ny * e.nz, prog.ntiles,
+                            program_acc(prog), prog.in_f64 != 0);
+    int rc = X3D_EUNSUPPORTED;
+    for (int i = 0; rc == X3D_EUNSUPPORTED && i < pick.count; ++i)
+        rc = launch_stage<T>(ctx, prog, dir, e.nx, e.ny, e.nz, pick.cfg[i]);
     for (int cfg = 0; rc == X3D_EUNSUPPORTED && cfg < kAllConfigs; ++cfg)
-        if (cfg != first && is_stage_cfg(cfg)) rc = launch_stage<T>(ctx, prog, dir, e.nx, e.ny, e.nz, cfg);
+        if (is_stage_cfg(cfg)) rc = launch_stage<T>(ctx, prog, dir, e.nx, e.ny, e.nz, cfg);
     return rc;
 }
 

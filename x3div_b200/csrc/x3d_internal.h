@@ -159,7 +159,8 @@ struct x3d_ctx_s {
     cudaGraph_t step_graph = nullptr;
     cudaGraphExec_t step_exec = nullptr;
     // kernel choice per (direction, grid, precision, operator-group size):
-    // filled by the autotuner, default_cfg otherwise
+    // filled by the autotuner; otherwise default_cfg, or where that is -1 the
+    // rule at default_cfgs (linesolve_chunk.h)
     std::map<std::string, int> tuned;
     // kernel choice per fused stage of the Euler step (transeq_x, div_y, ...),
     // filled by the autotuner; while stage_tuning is set, each stage run
@@ -167,7 +168,7 @@ struct x3d_ctx_s {
     std::map<std::string, int> stage_tuned;
     std::map<std::string, float> stage_ms;  // the tuned configuration's time (ms)
     bool stage_tuning = false;
-    int default_cfg = 0;
+    int default_cfg = -1;
     unsigned long long launches = 0;  // kernels of this library launched on the context
     int last_cfg = -1;                // configuration of the last line-solve launch (x3d_ctx_last_kernel)
     size_t elem() const { return precision == X3D_F32 ? 4 : 8; }
