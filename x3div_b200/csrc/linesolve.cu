@@ -572,7 +572,7 @@ int launch_group(x3d_ctx_s *ctx, int dir, const void *in, const x3d_op_s *const 
     if (it != ctx->tuned.end()) pick.cfg[0] = it->second;
     else if (ctx->default_cfg >= 0) pick.cfg[0] = ctx->default_cfg;
     else if (ops[0]->h.periodic)
-        pick = default_cfgs(fp32 ? 4 : 8, dir, ops[0]->h.n, (size_t)nx * ny * nz, 1, false, false);
+        pick = default_cfgs(fp32 ? 4 : 8, dir, nx, ny, nz, 1, nops, false, false, ctx->num_sms);
     int rc = X3D_EUNSUPPORTED;
     for (int i = 0; i < pick.count; ++i) {
         rc = run_cfg(ctx, pick.cfg[i], dir, in, ops, kinds, outs, nops, nx, ny, nz, fp32);

@@ -857,53 +857,110 @@ static int launch_stage_sel(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir
     }
 }
 
-// Measured on cubes of 16 to 384 points a side, every configuration on the
-// operator groups (one and six operators) and on the nine fused stages of a
-// step.  The lines:
-//   fields up to 4 MiB (96^3 FP32, 64^3 FP64): the launch ends before every SM
-//     is busy, so the short chunk, whose serial sweeps are half as long, wins
-//     (64^3 FP32, six y operators: 8.6 us on configuration 4, 17.9 on 0;
-//     momentum y 10.9 against 20.4);
-//   up to 16 MiB (128^3): wider tiles or a pair of lines a thread in FP32 (six
-//     y operators 18.2 on 14, 21.2 on 0), one CTA per tile in FP64;
-//   above: the kernels built for three CTAs per SM for plain programs (384^3
-//     FP64, six y operators: 673 us on 19, 1051 on 0; 256^3 FP32 y 113 on 20,
-//     127 on 0), pairs for accumulating FP32 y/z programs (256^3 momentum z 198
-//     on 14, 236 on 0) and 8-line tiles for FP64 x ones, whose three staged
-//     fields then fit more CTAs (256^3 momentum x 313 on 3, 460 on 0).
+// Which configuration an untuned program takes was measured on 41 boxes of 16
+// to 384 points a side, cubes and flat ones, both precisions: every
+// configuration on one and six operators and on the nine fused stages of a step.
+//
+// Fields above 24 MiB fill the SMs many times over, and the order is the same
+// for all of them: the kernels built for three CTAs per SM for plain programs
+// (384^3 FP64, six y operators: 673 us on 19, 1051 on 0; 256^3 FP32 y 113 on
+// 20, 127 on 0), pairs of lines a thread for FP32 y/z momentum (256^3 z 198 on
+// 14, 236 on 0), 8-line tiles for FP64 x programs that accumulate, whose three
+// staged fields then fit more CTAs (256^3 momentum x 313 on 3, 460 on 0).
+//
+// Below that what matters is how the tiles of a configuration divide into
+// waves, and no line through the sizes holds: stage_cost estimates each
+// configuration's time from its waves, and one that comes out at least a tenth
+// below the long-chunk default replaces it.  Over the measured launches the
+// pick is on average 4 % behind the fastest configuration and 19 % ahead of the
+// default (64^3 FP32, six y operators: 8.6 us on 4 against 17.9 on 0; 16 x 176
+// x 128 FP64 z, where the short chunk would take a second wave, stays on 0).
+//
 // The persistent configurations are left to the autotuner, although 17 is up
 // to 8 % ahead of 20: they claim tiles from the context's one counter, and an
 // untuned context may be moved between streams with launches in flight.
-DefaultCfgs default_cfgs(size_t es, int dir, int n, size_t points, int ntiles, bool acc, bool in64)
+struct StageShape {
+    int W, L, PR, regs, threads, ctas, per_sm;  // threads: 0 where it does not fit
+};
+
+// Tile width, chunk, resident CTAs of configuration cfg for a program.
+static StageShape stage_shape(int cfg, size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc,
+                              bool in64)
+{
+    const int n = dir == DX ? nx : (dir == DY ? ny : nz);
+    const int Llong = es == 4 ? 32 : 16;
+    StageShape s{};
+    s.PR = cfg == 14 ? 2 : 1;
+    s.regs = cfg >= 19 ? 80 : 128;
+    s.W = cfg == 3 || cfg == 5 || cfg == 19 ? 8 : (cfg == 1 || cfg == 4 || cfg == 14 ? 32 : 16);
+    s.L = cfg == 2 || cfg == 4 || cfg == 5 || cfg == 14 ? Llong / 2 : Llong;
+    const int C = (n + s.L - 1) / s.L, threads = C * s.W / s.PR;
+    if (threads % 32 || threads > (cfg >= 19 ? 256 : 512) || (cfg >= 19 && (acc || in64))) return s;
+    if (cfg == 14 && (es != 4 || dir == DX || nx % 2 || in64)) return s;
+    const size_t line = (size_t)s.W * (C * s.L + 2 * kHalo);
+    const size_t smem = line * (dir == DX ? (ntiles + 1) * es : ntiles * (in64 ? 8 : es)) + (size_t)2 * C * s.W * es +
+                        (size_t)nops * 4 * s.L * es * s.PR + 1024;
+    if (smem > (size_t)228 * 1024) return s;
+    s.threads = threads;
+    const long lines = dir == DX ? (long)ny * nz : nx;
+    const long tiles = (lines + s.W - 1) / s.W * (dir == DX ? 1 : (dir == DY ? nz : ny));
+    s.ctas = (int)std::min<long>(tiles, 1 << 30);
+    s.per_sm = std::max(1, std::min({65536 / (s.regs * threads), (int)(228 * 1024 / smem), 32, 2048 / threads}));
+    return s;
+}
+
+// Estimated microseconds of a launch of at most a few waves: a wave costs a
+// start, its operators one after another at a warp's own pace (a constant and
+// a slope in the chunk length) or, with r CTAs on an SM, at the SM's, and the
+// movement of its tiles.  The constants are a least-squares fit of the
+// logarithm to the measured launches up to 24 MiB (16 % rms).
+static double stage_cost(const StageShape &s, size_t es, int dir, int ntiles, int nops, bool acc, int num_sms)
+{
+    const bool f = es == 4, x = dir == DX;
+    const double op0 = f ? 0.2595 : 1.03, opL = f ? 0.06694 : 0.04398, issue = f ? 0.007064 : 0.01147;
+    const double start = f ? 0.2606 : 0.6114, move = f ? 1.011 : 0.007316;
+    const double kx = x ? 1.113 : 1.0, ka = acc ? 1.254 : 1.0, pair = s.PR == 2 ? 1.104 : 1.0;
+    const double alone = (op0 + opL * s.L * (s.PR == 2 ? 1.15 : 1.0)) * nops * kx * ka;
+    const double a4 = alone * alone * alone * alone;
+    auto wave = [&](int r) {
+        const double shared = r * (s.threads / 32) * s.L * nops * issue * kx * ka * pair * (s.W == 8 ? 1.125 : 1.0);
+        return start * kx + (x ? 0.0475 * s.W * ntiles : 0.0) +
+               std::sqrt(std::sqrt(a4 + shared * shared * shared * shared)) * (s.PR == 2 && acc ? 1.217 : 1.0) +
+               move * 1e-5 * r * s.threads * s.L * s.PR * (double)es;
+    };
+    const int slots = num_sms * s.per_sm, full = s.ctas / slots, rest = s.ctas - full * slots;
+    return 2.0 + full * wave(s.per_sm) + (rest ? wave((rest + num_sms - 1) / num_sms) : 0.0);
+}
+
+DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
+                         int num_sms)
 {
     const bool f32 = es == 4;
-    const size_t bytes = points * es;
-    const bool small = bytes <= (size_t)4 << 20, mid = bytes <= (size_t)16 << 20;
-    if (dir == DX) {
-        if (small) return {5, {2, 4, 5, 1, 0}};
-        if (acc) {
-            if (f32 && mid) return {3, {2, 5, 0}};
-            if (f32) return {2, {0, 3}};
-            return {3, {3, 1, 0}};
+    if ((size_t)nx * ny * nz * es > (size_t)24 << 20) {
+        if (dir == DX) {
+            if (acc) return f32 ? DefaultCfgs{2, {0, 3}} : DefaultCfgs{2, {3, 0}};
+            if (f32 && ntiles > 1) return {3, {5, 19, 0}};
+            return {3, {19, 20, 0}};
         }
-        if (f32 && ntiles > 1) return {4, {5, 2, 19, 0}};
-        if (f32 && (mid || n < 256)) return {4, {20, 19, 0, 1}};
-        return {4, {19, 20, 3, 0}};
+        if (acc) return f32 && nops == 6 ? DefaultCfgs{2, {14, 0}} : DefaultCfgs{2, {0, 3}};
+        if (in64) return {1, {0}};
+        return {3, {20, 19, 0}};
     }
-    if (small) return {5, {4, 2, 1, 0, 5}};
-    if (acc) {
-        if (f32 && mid) return {3, {1, 14, 0}};
-        if (f32) return {3, {14, 1, 0}};
-        if (mid) return {3, {1, 0, 3}};
-        if (ntiles < 3 && n > 256) return {3, {3, 0, 1}};
-        return {3, {0, 3, 1}};
+    static const int cand[] = {0, 1, 2, 3, 4, 5, 14, 19, 20};
+    int base = -1, best = -1;
+    double tbase = 0.0, tbest = 0.0;
+    for (const int cfg : cand) {
+        const StageShape s = stage_shape(cfg, es, dir, nx, ny, nz, ntiles, nops, acc, in64);
+        if (!s.threads) continue;
+        // 32 row copies issued by one thread: only where nothing else fits
+        if (cfg == 4 && dir == DX && base >= 0) continue;
+        const double t = stage_cost(s, es, dir, ntiles, nops, acc, num_sms);
+        if (base < 0) base = cfg, tbase = t;
+        if (best < 0 || t < tbest) best = cfg, tbest = t;
     }
-    if (in64) {
-        if (mid) return {2, {1, 0}};
-        return {2, {0, 3}};
-    }
-    if (f32 && mid) return {4, {14, 1, 20, 0}};
-    return {3, {20, 19, 0}};
+    if (base < 0) return {1, {0}};
+    if (tbest < 0.9 * tbase) return {2, {best, base}};
+    return {1, {base}};
 }
 
 template <typename T>

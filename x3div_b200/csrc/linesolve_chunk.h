@@ -75,16 +75,16 @@ template <typename T>
 int launch_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, int nx, int ny, int nz,
                  int cfg);
 
-// Up to kMaxDefaultCfgs configurations for a program that the autotuner has not
-// timed, best first, by the rule at default_cfgs (linesolve_chunk.cu).
-constexpr int kMaxDefaultCfgs = 5;
+// Configurations for a program that the autotuner has not timed, best first, by
+// the rule at default_cfgs (linesolve_chunk.cu).
 struct DefaultCfgs {
-    int count, cfg[kMaxDefaultCfgs];
+    int count, cfg[3];
 };
-// es: element bytes of the context; n: points a line; points: of the field;
-// ntiles: staged inputs; acc: the program accumulates or flushes other than
-// plainly; in64: FP64 inputs of an FP32 program.
-DefaultCfgs default_cfgs(size_t es, int dir, int n, size_t points, int ntiles, bool acc, bool in64);
+// es: element bytes of the context; ntiles, nops: staged inputs and operators;
+// acc: the program accumulates or flushes other than plainly; in64: FP64 inputs
+// of an FP32 program.
+DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
+                         int num_sms);
 
 // Whether a program needs the kernels with the accumulator and every flush form.
 template <typename T>

@@ -122,19 +122,24 @@ static int tune_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, cons
     return X3D_OK;
 }
 
-// Runs one program with its tuned (or the default) configuration, then, if
-// that one cannot take the grid, the others in order.
+// The configurations an untuned stage tries first.
 template <typename T>
-static int run_program(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, const std::string &name, Ext e)
+static DefaultCfgs stage_default(const x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, Ext e)
+{
+    if (is_stage_cfg(ctx->default_cfg)) return {1, {ctx->default_cfg}};
+    return default_cfgs(sizeof(T), dir, e.nx, e.ny, e.nz, prog.ntiles, prog.nops, program_acc(prog), prog.in_f64 != 0,
+                        ctx->num_sms);
+}
+
+// Runs one program with its tuned (or the stage's default) configuration,
+// then, if that one cannot take the grid, the others in order.
+template <typename T>
+static int run_program(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, const std::string &name, Ext e,
+                       DefaultCfgs pick)
 {
     if (ctx->stage_tuning) return tune_stage<T>(ctx, prog, dir, name.c_str(), e);
     const auto it = ctx->stage_tuned.find(name);
-    DefaultCfgs pick{1, {0}};
-    if (it != ctx->stage_tuned.end()) pick.cfg[0] = it->second;
-    else if (is_stage_cfg(ctx->default_cfg)) pick.cfg[0] = ctx->default_cfg;
-    else
-        pick = default_cfgs(sizeof(T), dir, prog.ops[0].op.n, (size_t)e.nx * e.ny * e.nz, prog.ntiles,
-                            program_acc(prog), prog.in_f64 != 0);
+    if (it != ctx->stage_tuned.end()) pick = {1, {it->second}};
     int rc = X3D_EUNSUPPORTED;
     for (int i = 0; rc == X3D_EUNSUPPORTED && i < pick.count; ++i)
         rc = launch_stage<T>(ctx, prog, dir, e.nx, e.ny, e.nz, pick.cfg[i]);
@@ -146,8 +151,12 @@ static int run_program(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir, con
 // Runs a stage: one launch, or, where the autotuner found it faster, one
 // launch per part of split_by_inputs (stages "<name>.1", "<name>.2", ...).
 // While tuning, times both forms and records the choice as "<name>.parts".
+// Untuned, the parts take the whole stage's default (whole: the program it is
+// read from, where that is not prog_in), so that a stage gives the same bits in
+// either form.
 template <typename T>
-static int run_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int dir, const char *cname, Ext e)
+static int run_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int dir, const char *cname, Ext e,
+                     const StageProgram<T> *whole = nullptr)
 {
     const TraceRange trace(cname);
     const std::string name = stage_key(ctx, cname, e);
@@ -157,15 +166,16 @@ static int run_stage(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int dir, co
     const int nparts = split_by_inputs<T>(prog, part);
     const auto it = ctx->stage_tuned.find(name + ".parts");
     const bool split = nparts > 1 && !ctx->stage_tuning && it != ctx->stage_tuned.end() && it->second == nparts;
+    const DefaultCfgs pick = stage_default<T>(ctx, whole ? *whole : prog, dir, e);
     int rc = X3D_OK;
     if (!split) {
-        rc = run_program<T>(ctx, prog, dir, name, e);
+        rc = run_program<T>(ctx, prog, dir, name, e, pick);
         if (rc || !ctx->stage_tuning || nparts < 2) return rc;
     }
     float total = 0.f;
     for (int q = 0; q < nparts && !rc; ++q) {
         const std::string pn = name + "." + std::to_string(q + 1);
-        rc = run_program<T>(ctx, part[q], dir, pn, e);
+        rc = run_program<T>(ctx, part[q], dir, pn, e, pick);
         if (!rc && ctx->stage_tuning) total += ctx->stage_ms[pn];
     }
     if (ctx->stage_tuning) {
@@ -243,8 +253,11 @@ static int transeq_dir(x3d_ctx_s *ctx, int d, void *const du[3], const void *con
     }
     if (split || ctx->stage_tuning) {
         const std::string nb = std::string(names[d]) + ".b", na = std::string(names[d]) + ".a";
-        rc = run_stage<T>(ctx, transeq_program<T>(ctx, d, &o2, 1, du, u, add, unew, dt), d, nb.c_str(), e);
-        if (!rc) rc = run_stage<T>(ctx, transeq_program<T>(ctx, d, first, 2, du, u, add, unew, dt), d, na.c_str(), e);
+        const StageProgram<T> whole = transeq_program<T>(ctx, d, all, 3, du, u, add, unew, dt);
+        rc = run_stage<T>(ctx, transeq_program<T>(ctx, d, &o2, 1, du, u, add, unew, dt), d, nb.c_str(), e, &whole);
+        if (!rc)
+            rc = run_stage<T>(ctx, transeq_program<T>(ctx, d, first, 2, du, u, add, unew, dt), d, na.c_str(), e,
+                              &whole);
         if (rc && !(ctx->stage_tuning && rc == X3D_EUNSUPPORTED)) return rc;
         if (ctx->stage_tuning) {
             const float t3 = ctx->stage_ms[name];
