@@ -274,3 +274,41 @@ def test_nonperiodic_poisson_matches_oracle(oracle, torch_cuda, prec, shape, per
         ref = oracle.poisson_bc(np.asfortranarray(g), lengths, per)
         assert rel_err(to_host(rhs), ref) < 1e-12, (shape, per, seed)
     ctx.close()
+
+
+# mirrored lengths with own transforms (nx / 2, nz and, with walls in y, ny):
+# every radix pattern the halves go through (a single radix, 8s, 4, 2, 3s, the
+# separate split pass of nx / 2 = 64), partial last tiles of rows and lanes,
+# and walls in one, two and three directions
+@pytest.mark.parametrize("shape,per", [((9, 10, 12), (False, True, True)), ((65, 11, 16), (False, True, True)),
+                                       ((25, 7 + 1, 8), (False, True, True)), ((24, 9, 12), (True, False, True)),
+                                       ((16, 33, 24), (True, False, True)), ((48, 129, 16), (True, False, True)),
+                                       ((32, 11, 9), (True, True, False)), ((16, 9, 97), (True, True, False)),
+                                       ((17, 13, 12), (False, False, True)), ((33, 17, 25), (False, False, False)),
+                                       ((128, 65, 33), (True, False, False)), ((16, 385, 8), (True, False, True))])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_nonperiodic_poisson_on_halves(oracle, torch_cuda, shape, per, offset):
+    """The solve that transforms the first half of each mirrored line, against
+    the oracle's mirrored box; offset: a right-hand side one element into its
+    allocation, which goes through the mirrored box in memory, before and
+    after an aligned one on the same context."""
+    torch = torch_cuda
+    from x3div_b200 import Context, to_host
+    lengths = (2 * np.pi, 1.5, 3.0)
+    bc = []
+    for p_ in per:
+        bc += [0, 0] if p_ else [1, 1]
+    ctx = Context(*shape, lengths=lengths, bc=tuple(bc))
+    pshape = tuple(n if p_ else n - 1 for n, p_ in zip(shape, per))
+    for seed, off in ((3, offset), (4, 0), (5, offset)):
+        g = np.random.default_rng(seed).standard_normal(pshape)
+        flat = torch.empty(g.size + off, dtype=torch.float64, device="cuda")
+        rhs = flat[off:].view(pshape[::-1])
+        rhs.copy_(torch.from_numpy(np.ascontiguousarray(g.transpose(2, 1, 0))))
+        n0 = ctx.launch_count()
+        ctx.poisson(rhs)
+        ctx.sync()
+        if not off:  # x, z, x and, with walls in y, two own y transforms
+            assert ctx.launch_count() - n0 == (3 if per[1] else 5)
+        assert rel_err(to_host(rhs), oracle.poisson_bc(np.asfortranarray(g), lengths, per)) < 1e-12, (shape, per, seed)
+    ctx.close()

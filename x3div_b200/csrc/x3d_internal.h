@@ -123,6 +123,13 @@ struct x3d_ctx_s {
     // that layout, and back.  d_xft_tw: e^{-2 pi i t / (nx/2)}, t < nx/2, then
     // e^{-2 pi i k / nx}, k <= nx/2 (complex).
     double *d_xft_tw = nullptr;
+    // A mirrored box solved on its first halves (poisson_solve_halves): the
+    // spectrum of the unmirrored planes and rows, the tables of the cosine
+    // transforms along y where y is mirrored (see k_dct_y), and else the y plan.
+    void *half_spectrum = nullptr;
+    double *d_yft_tw = nullptr;
+    cufftHandle plan_yh = 0;
+    bool plan_yh_ready = false;
     cufftHandle plan_y = 0;
     bool plan_y_ready = false;
     // batched 1-D z transforms of one rank's block of the half spectrum, for
