@@ -135,6 +135,26 @@ int make_jobs(x3d_batch_s *b, std::vector<BatchJob<T>> &jobs, size_t *tile_cap_o
                     fb.kinds[k] = kinds[k];
                     fb.outs[k] = J.out[k];
                 }
+                // the shifted twins: derpv and interpv as second outputs of
+                // dervp and intervp, where x rows can be stored as vectors
+                for (int k = 0, kept = 0, n0 = J.nops; k < n0; ++k) {
+                    int vp = -1;
+                    bool twice = false;  // the order of writes to one output stays as listed
+                    for (int j = 0; j < nops_per_dir; ++j) twice = twice || (j != k && fb.outs[j] == fb.outs[k]);
+                    for (int j = 0; j < kept && vp < 0 && !twice; ++j)
+                        if (!J.shift_out[j] && shifted_twin<T>(J.op[j], J.kind[j], J.op[k], J.kind[k]) &&
+                            (d != DX || reinterpret_cast<uintptr_t>(J.out[k]) % 16 == 0))
+                            vp = j;
+                    if (vp >= 0) {
+                        J.shift_out[vp] = J.out[k];
+                        --J.nops;
+                    } else {
+                        J.op[kept] = J.op[k];
+                        J.kind[kept] = J.kind[k];
+                        J.out[kept] = J.out[k];
+                        ++kept;
+                    }
+                }
                 if (whole) b->points += (long long)nops_per_dir * dims[0] * dims[1] * dims[2];
                 const int sd = b->box_shape[i] * 3 + d;
                 const int L = L_force > 0 ? L_force : (b->choice_L[sd] > 0 ? b->choice_L[sd] : kChunkLong<T>);

@@ -569,6 +569,59 @@ __device__ __forceinline__ void flush_yz(const FlushArgs<T> &fa, const V (&res)[
     }
 }
 
+// Writes a solved y/z chunk one point further along its periodic line
+// (StageOp::shift_out): obase is point cs, and the line's last point, which
+// the thread of the last chunk holds, goes to its first.
+template <typename T, typename V, int L>
+__device__ __forceinline__ void flush_yz_shifted(void *shift_out, const V (&res)[L], size_t obase, int cs,
+                                                 size_t ostride, int nv, bool last)
+{
+    T *const out = static_cast<T *>(shift_out);
+    T *dst = out + obase + ostride;
+    if (!last) {
+#pragma unroll
+        for (int j = 0; j < L; ++j, dst += ostride) *reinterpret_cast<V *>(dst) = res[j];
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < L; ++j, dst += ostride) {
+        if (j + 1 < nv) *reinterpret_cast<V *>(dst) = res[j];
+        else if (j + 1 == nv) *reinterpret_cast<V *>(out + obase - (size_t)cs * ostride) = res[j];
+    }
+}
+
+// The same for a tile of x lines from its staging rows: element i of a row is
+// read from i - 1.  Vectors of 16 bytes (VEC: n and the output are whole ones)
+// take their first element from the lane before.
+template <typename T, bool VEC>
+__device__ __forceinline__ void flush_rows_shifted(void *shift_out, const T *out_s, long l0, int rows, int pitch,
+                                                   int n)
+{
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int rr = threadIdx.x >> 5; rr < rows; rr += nw) {
+        const T *row = out_s + (size_t)rr * pitch;
+        T *dst = static_cast<T *>(shift_out) + (size_t)(l0 + rr) * n;
+        if constexpr (VEC) {
+            using VT = typename Vec4<T>::type;
+            constexpr int N = Vec4<T>::N;
+            const int nvec = n / N;
+            for (int q0 = 0; q0 < nvec; q0 += 32) {
+                const int q = q0 + lane;
+                VT v = *reinterpret_cast<const VT *>(row + (q < nvec ? q : 0) * N);
+                T *e = reinterpret_cast<T *>(&v);
+                T prev = __shfl_up_sync(0xffffffffu, e[N - 1], 1);
+                if (lane == 0) prev = row[q ? q * N - 1 : n - 1];
+#pragma unroll
+                for (int i = N - 1; i > 0; --i) e[i] = e[i - 1];
+                e[0] = prev;
+                if (q < nvec) *reinterpret_cast<VT *>(dst + q * N) = v;
+            }
+        } else {
+            for (int i = lane; i < n; i += 32) dst[i] = row[i ? i - 1 : n - 1];
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Host side.
 

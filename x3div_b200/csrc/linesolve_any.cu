@@ -93,6 +93,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
             if (so.flush && live) flush_yz<T, T, L, true>(flush_args(so), acc, obase, stride, nv);
         } else {
             if (so.flush && live) flush_yz<T, T, L, false>(flush_args(so), r, obase, stride, nv);
+            if (so.shift_out && live) flush_yz_shifted<T, T, L>(so.shift_out, r, obase, cs, stride, nv, c == C - 1);
         }
     }
 }
@@ -233,6 +234,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
             else flush_rows_any<T, T, true>(so, out_s, g0, rows, pitch, n);
         } else {
             flush_rows_any<T, T, false>(so, out_s, g0, rows, pitch, n);
+            if (so.shift_out) flush_rows_shifted<T, false>(so.shift_out, out_s, l0, rows, pitch, n);
         }
     }
 }

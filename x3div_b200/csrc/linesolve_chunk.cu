@@ -225,6 +225,8 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : kStageThreads<T, L, PR>, OCC)
                 if (so.flush && live) flush_yz<T, V, L, true>(flush_args(so), acc, obase, ostride, nv);
             } else {
                 if (so.flush && live) flush_yz<T, V, L, false>(flush_args(so), r, obase, ostride, nv);
+                if (so.shift_out && live)
+                    flush_yz_shifted<T, V, L>(so.shift_out, r, obase, cs, ostride, nv, c == C - 1);
             }
         }
         if (!PERSIST) break;
@@ -595,6 +597,9 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
                 if (so.flush) flush_x_staged<T, L, true>(flush_args(so), acc, out_s, l, l0, rows, pitch, n, cs, nv);
             } else {
                 if (so.flush) flush_x_staged<T, L, false>(flush_args(so), r, out_s, l, l0, rows, pitch, n, cs, nv);
+                // from the staging rows, which the next operator writes only
+                // after its solve's barriers
+                if (so.shift_out) flush_rows_shifted<T, true>(so.shift_out, out_s, l0, rows, pitch, n);
             }
         }
         if (!PERSIST) break;
@@ -643,7 +648,8 @@ static bool whole_vectors(const StageProgram<T> &p, int dir, int nx)
         if (!al16(p.in[ti])) return false;
     for (int k = 0; k < p.nops && dir == DX; ++k) {
         const StageOp<T> &so = p.ops[k];
-        if (so.flush && (!al16(so.out) || !al16(so.base) || !al16(so.out2) || !al16(so.base2))) return false;
+        if (so.flush && (!al16(so.out) || !al16(so.base) || !al16(so.out2) || !al16(so.base2) || !al16(so.shift_out)))
+            return false;
     }
     return true;
 }
@@ -709,7 +715,8 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
             if (dir == DX || nx % 2) return X3D_EUNSUPPORTED;
             for (int k = 0; k < prog.nops; ++k) {
                 const StageOp<T> &so = prog.ops[k];
-                if (so.flush && (!al8(so.out) || !al8(so.base) || !al8(so.out2) || !al8(so.base2)))
+                if (so.flush &&
+                    (!al8(so.out) || !al8(so.base) || !al8(so.out2) || !al8(so.base2) || !al8(so.shift_out)))
                     return X3D_EUNSUPPORTED;
             }
         } else if (dir == DX) {
@@ -968,11 +975,26 @@ StageProgram<T> plain_program(const T *in, const LineOp<T> *const *ops, const in
                               void *const *outs, int nops)
 {
     StageProgram<T> p{};
-    p.nops = nops;
     p.ntiles = 1;
     p.in[0] = in;
+    // twin[k] = j: operator k is j's shifted twin, written by j's solve (one
+    // twin a solve; not where the list names an output twice, whose order of
+    // writes it would change)
+    int twin[kMaxStageOps];
+    bool taken[kMaxStageOps] = {};
     for (int k = 0; k < nops; ++k) {
-        StageOp<T> &so = p.ops[k];
+        twin[k] = -1;
+        bool twice = false;
+        for (int j = 0; j < nops; ++j) twice = twice || (j != k && outs[j] == outs[k]);
+        for (int j = 0; j < nops && twin[k] < 0 && !twice; ++j)
+            if (j != k && !taken[j] && shifted_twin<T>(*ops[j], kinds[j], *ops[k], kinds[k])) {
+                twin[k] = j;
+                taken[j] = true;
+            }
+    }
+    for (int k = 0; k < nops; ++k) {
+        if (twin[k] >= 0) continue;
+        StageOp<T> &so = p.ops[p.nops++];
         so.op = *ops[k];
         so.kind = kinds[k];
         so.src_a = 0;
@@ -987,6 +1009,8 @@ StageProgram<T> plain_program(const T *in, const LineOp<T> *const *ops, const in
         so.sign = 1.0;
         so.scale2 = 0.0;
         so.out_f64 = 0;
+        for (int j = 0; j < nops; ++j)
+            if (twin[j] == k) so.shift_out = outs[j];
     }
     return p;
 }
@@ -1068,6 +1092,34 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                         }
                     }
                 }
+                if (J.shift_out[k]) {
+                    // one point on: the chunk's first point is the end of the
+                    // chunk before, passed through the scratch that held the
+                    // forward ends (read before the solve's second barrier)
+                    T end = T(0);
+#pragma unroll
+                    for (int j = 0; j < L; ++j)
+                        if (j + 1 == nv) end = r[j];
+                    sc.fz[q] = end;
+                    __syncthreads();
+                    T prev = sc.fz[(c ? c - 1 : C - 1) * W + l];
+                    if (active && l < rows) {
+                        T *dst = J.shift_out[k] + (size_t)(l0 + l) * n + cs;
+#pragma unroll
+                        for (int j = 0; j < L; j += V) {
+                            if (j < nv) {
+                                VT qv;
+                                T *e = reinterpret_cast<T *>(&qv);
+                                e[0] = prev;
+#pragma unroll
+                                for (int v = 1; v < V; ++v) e[v] = r[j + v - 1];
+                                prev = r[j + V - 1];
+                                *reinterpret_cast<VT *>(dst + j) = qv;
+                            }
+                        }
+                    }
+                    __syncthreads();  // before the next operator writes the scratch
+                }
                 continue;
             }
             if (active && l < rows) {
@@ -1088,6 +1140,7 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                            (uint32_t)(n * sizeof(T)));
                 bulk_commit();
             }
+            if (J.shift_out[k]) flush_rows_shifted<T, true>(J.shift_out[k], out_s, l0, rows, J.pitch, n);
         }
     } else {
         const T *col = tile + (size_t)(J.halo + cs - 4) * W + l;  // points cs-4 .. cs+L+3
@@ -1120,6 +1173,8 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                         dst += ostride;
                     }
                 }
+                if (J.shift_out[k])
+                    flush_yz_shifted<T, T, L>(J.shift_out[k], r, obase, cs, ostride, nv, c == C - 1);
             }
         }
     }

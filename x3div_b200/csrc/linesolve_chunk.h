@@ -36,6 +36,9 @@ struct StageOp {
     // the tile's inputs are requested.
     short base2_tile;
     short prefetch_base;
+    // Plain programs: a second output, the solve one point further along the
+    // line (shift_out[i + 1] = x[i], periodic), or null; see shifted_twin.
+    void *shift_out;
     // Set by launch_stage: the response entries the fixes of a full chunk
     // use (see chunk_solve_resp).
     int keep;
@@ -86,6 +89,19 @@ struct DefaultCfgs {
 DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
                          int num_sms);
 
+// The pressure-to-velocity operators (derpv, interpv) take the stencil of their
+// velocity-to-pressure twins one point back, r_pv[i] = r_vp[i - 1], and a
+// periodic operator's matrix is circulant, so on one input the solve of pv is
+// that of vp one point on: where a group applies both, one solve is written
+// twice.  Whether pv is vp's shifted twin in that sense.
+template <typename T>
+inline bool shifted_twin(const LineOp<T> &vp, int vp_kind, const LineOp<T> &pv, int pv_kind)
+{
+    if (!(vp_kind == DERVP && pv_kind == DERPV) && !(vp_kind == INTVP && pv_kind == INTPV)) return false;
+    return vp.circ && pv.circ && vp.n == pv.n && vp.alfa == pv.alfa && vp.a == pv.a && vp.b == pv.b && vp.c == pv.c &&
+           vp.d == pv.d;
+}
+
 // Whether a program needs the kernels with the accumulator and every flush form.
 template <typename T>
 inline bool program_acc(const StageProgram<T> &p)
@@ -114,6 +130,7 @@ struct BatchJob {
     CUtensorMap tmap;  // y/z input map
     const T *in;
     T *out[kMaxStageOps];
+    T *shift_out[kMaxStageOps];  // as StageOp::shift_out
     LineOp<T> op[kMaxStageOps];
     int kind[kMaxStageOps];
     int nops, dir, n, nx, ny, nz;
