@@ -4,6 +4,7 @@
 #include <cmath>
 
 #include "ptx.cuh"
+#include "launch_pdl.h"
 #include "x3d_internal.h"
 
 namespace x3d {
@@ -18,6 +19,8 @@ static unsigned grid_for(const x3d_ctx_s *ctx, size_t n, int bs)
 template <typename T>
 __global__ void k_axpy3(T *u, T *v, T *w, const T *du, const T *dv, const T *dw, T alpha, size_t n)
 {
+    pdl_trigger();
+    pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         u[i] = alpha * du[i] + u[i];
         v[i] = alpha * dv[i] + v[i];
@@ -28,6 +31,8 @@ __global__ void k_axpy3(T *u, T *v, T *w, const T *du, const T *dv, const T *dw,
 template <typename T>
 __global__ void k_sub3(T *u, T *v, T *w, const T *a, const T *b, const T *c, size_t n)
 {
+    pdl_trigger();
+    pdl_wait();
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         u[i] = u[i] - a[i];
         v[i] = v[i] - b[i];
@@ -164,6 +169,15 @@ __global__ void k_scale_y(T *t, const double *ppy, int nx, int ny, size_t n)
         return cuda_check(ctx, cudaGetLastError(), #kern);                                \
     } while (0)
 
+// The two updates of the driver's own time loop, between its other launches.
+#define X3D_LAUNCH_PDL(kern, n, ...)                                                                        \
+    do {                                                                                                    \
+        const int bs_ = 256;                                                                                \
+        ++ctx->launches;                                                                                    \
+        return cuda_check(ctx, launch_pdl(kern, grid_for(ctx, (n), bs_), bs_, 0, ctx->stream, __VA_ARGS__), \
+                          #kern);                                                                           \
+    } while (0)
+
 int launch_copy(x3d_ctx_s *ctx, void *dst, const void *src, size_t bytes)
 {
     if (dst == src) return X3D_OK;
@@ -175,9 +189,9 @@ int launch_axpy3(x3d_ctx_s *ctx, bool fp32, void *u, void *v, void *w, const voi
                  const void *dv, const void *dw, double alpha, size_t n)
 {
     if (fp32)
-        X3D_LAUNCH(k_axpy3<float>, n, (float *)u, (float *)v, (float *)w, (const float *)du,
+        X3D_LAUNCH_PDL(k_axpy3<float>, n, (float *)u, (float *)v, (float *)w, (const float *)du,
                    (const float *)dv, (const float *)dw, (float)alpha, n);
-    X3D_LAUNCH(k_axpy3<double>, n, (double *)u, (double *)v, (double *)w, (const double *)du,
+    X3D_LAUNCH_PDL(k_axpy3<double>, n, (double *)u, (double *)v, (double *)w, (const double *)du,
                (const double *)dv, (const double *)dw, alpha, n);
 }
 
@@ -185,9 +199,9 @@ int launch_sub3(x3d_ctx_s *ctx, bool fp32, void *u, void *v, void *w, const void
                 const void *c, size_t n)
 {
     if (fp32)
-        X3D_LAUNCH(k_sub3<float>, n, (float *)u, (float *)v, (float *)w, (const float *)a,
+        X3D_LAUNCH_PDL(k_sub3<float>, n, (float *)u, (float *)v, (float *)w, (const float *)a,
                    (const float *)b, (const float *)c, n);
-    X3D_LAUNCH(k_sub3<double>, n, (double *)u, (double *)v, (double *)w, (const double *)a,
+    X3D_LAUNCH_PDL(k_sub3<double>, n, (double *)u, (double *)v, (double *)w, (const double *)a,
                (const double *)b, (const double *)c, n);
 }
 

@@ -14,6 +14,7 @@
 // 256 threads for plain programs, 80 registers a thread), and their copies,
 // solves and stores overlap.
 #include "chunk_solve.cuh"
+#include "launch_pdl.h"
 #include "linesolve_chunk.h"
 #include "ptx.cuh"
 #include "tile_copy.cuh"
@@ -37,6 +38,11 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
     const size_t stride = dir == DY ? (size_t)nx : (size_t)nx * ny;
     const size_t plane = (size_t)x0 + (dir == DY ? (size_t)nx * ny * o : (size_t)nx * o);
     const int cols = min(W, nx - x0);
+    pdl_trigger();
+    T *resp_s = reinterpret_cast<T *>(smem_raw + prog.ntiles * tile_bytes +
+                                      (((size_t)2 * nt * sizeof(T) + 15) & ~(size_t)15));
+    load_resp<T, L>(prog, resp_s);
+    pdl_wait();
     for (int ti = 0; ti < prog.ntiles; ++ti) {
         const TI *src = reinterpret_cast<const TI *>(prog.in[ti]) + plane;
         TI *tp = reinterpret_cast<TI *>(smem_raw + ti * tile_bytes);
@@ -48,8 +54,6 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
                                      src + (size_t)(h < kHalo ? n - kHalo + h : h - kHalo) * stride + x);
         }
     }
-    T *resp_s = reinterpret_cast<T *>(smem_raw + prog.ntiles * tile_bytes + (((size_t)2 * nt * sizeof(T) + 15) & ~(size_t)15));
-    load_resp<T, L>(prog, resp_s);
     const ChunkScratch<T> sc = carve_scratch<T>(smem_raw + prog.ntiles * tile_bytes, nt, 1);
     cp_async_wait_all();
     __syncthreads();
@@ -157,6 +161,11 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
     const int t = threadIdx.x, nt = blockDim.x;
     const long l0 = (long)blockIdx.x * W;
     const int rows = (int)min((long)W, nlines - l0);
+    pdl_trigger();
+    T *resp_s = reinterpret_cast<T *>(smem_raw + prog.ntiles * tile_bytes +
+                                      (((size_t)2 * nt * sizeof(T) + 15) & ~(size_t)15));
+    load_resp<T, L>(prog, resp_s);
+    pdl_wait();
     for (int ti = 0; ti < prog.ntiles; ++ti) {
         T *tp = reinterpret_cast<T *>(smem_raw + ti * tile_bytes);
         const T *src = prog.in[ti] + (size_t)l0 * n;
@@ -167,8 +176,6 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
                                 src + (size_t)rr * n + (h < kHalo ? n - kHalo + h : h - kHalo));
         }
     }
-    T *resp_s = reinterpret_cast<T *>(smem_raw + prog.ntiles * tile_bytes + (((size_t)2 * nt * sizeof(T) + 15) & ~(size_t)15));
-    load_resp<T, L>(prog, resp_s);
     const ChunkScratch<T> sc = carve_scratch<T>(smem_raw + prog.ntiles * tile_bytes, nt, 1);
     T *out_s = resp_s + prog.nops * 4 * L;
     cp_async_wait_all();
@@ -261,8 +268,8 @@ int launch_stage_any(x3d_ctx_s *ctx, const StageProgram<T> &prog, bool acc, int 
         if (smem + 1024 > ctx->smem_optin || grid > 0x7fffffffL) return (int)X3D_EUNSUPPORTED;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        kern<<<(unsigned)grid, threads, smem, ctx->stream>>>(prog, args...);
-        return cuda_check(ctx, cudaGetLastError(), "ls_any launch");
+        return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, prog, args...),
+                          "ls_any launch");
     };
     if (dir == DX) {
         int pitch = C * L + 2 * kHalo;

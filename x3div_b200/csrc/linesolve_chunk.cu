@@ -44,6 +44,7 @@
 #include <type_traits>
 
 #include "chunk_solve.cuh"
+#include "launch_pdl.h"
 #include "linesolve_chunk.h"
 #include "ptx.cuh"
 #include "x3d_internal.h"
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : kStageThreads<T, L, PR>, OCC)
     const size_t slot_bytes = (size_t)prog.ntiles * tile_bytes;
     V *resp_s = reinterpret_cast<V *>(smem_raw + (PERSIST ? 2 : 1) * slot_bytes +
                                       (((size_t)2 * C * W * sizeof(T) + 15) & ~(size_t)15));
+    pdl_trigger();
     load_resp<V, L>(prog, resp_s);
     if (t == 0) {
         mbar_init(&bars[0], 1);
@@ -150,6 +152,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : kStageThreads<T, L, PR>, OCC)
     const int cs = c * L;
     const int nv = min(L, n - cs);
     const size_t ostride = dir == DY ? (size_t)nx : (size_t)nx * ny;
+    pdl_wait();
     long tile = blockIdx.x;
     if (t == 0) {
         if (PERSIST) s_tile[0] = tile = (long)atomicAdd(claim, 1ull);
@@ -487,6 +490,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
     const size_t slot_bytes = (size_t)prog.ntiles * tile_bytes;
     T *resp_s = reinterpret_cast<T *>(smem_raw + (PERSIST ? 2 : 1) * slot_bytes +
                                       (((size_t)2 * C * W * sizeof(T) + 15) & ~(size_t)15));
+    pdl_trigger();
     load_resp<T, L>(prog, resp_s);
     if (t == 0) {
         mbar_init(&bars[0], 1);
@@ -517,6 +521,7 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
         smem_raw + ((reinterpret_cast<unsigned char *>(resp_s + prog.nops * 4 * L) - smem_raw + 127) & ~(size_t)127));
     const int cs = c * L;
     const int nv = min(L, n - cs);
+    pdl_wait();
     long tile = blockIdx.x;
     if (t == 0) {
         if (PERSIST) s_tile[0] = tile = (long)atomicAdd(claim, 1ull);
@@ -744,8 +749,9 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                 if (rc) return rc;
             }
             ++ctx->launches;
-            kern<<<grid, threads, smem, st>>>(prog, nlines, pitch, tile, ntiles, ctx->d_claim, ctx->d_err);
-            return cuda_check(ctx, cudaGetLastError(), "ls_stage_x launch");
+            return cuda_check(ctx, launch_pdl(kern, grid, threads, smem, st, prog, nlines, pitch, tile, ntiles,
+                                              ctx->d_claim, ctx->d_err),
+                              "ls_stage_x launch");
         }
         auto enc = encode_tiled();
         const size_t esi = in64 ? sizeof(double) : es;  // staged element bytes
@@ -805,9 +811,9 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
             if (rc) return rc;
         }
         ++ctx->launches;
-        kern<<<grid, threads, smem, st>>>(maps, prog, nx, ny, dir, box_n, nb, tma_halo, tile, ntiles, ctx->d_claim,
-                                          ctx->d_err);
-        return cuda_check(ctx, cudaGetLastError(), "ls_stage_yz launch");
+        return cuda_check(ctx, launch_pdl(kern, grid, threads, smem, st, maps, prog, nx, ny, dir, box_n, nb, tma_halo,
+                                          tile, ntiles, ctx->d_claim, ctx->d_err),
+                          "ls_stage_yz launch");
 
     }
 }

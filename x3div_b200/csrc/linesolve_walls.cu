@@ -19,6 +19,7 @@
 
 #include "chunk_solve.cuh"
 #include "der_closure.cuh"
+#include "launch_pdl.h"
 #include "linesolve_chunk.h"
 #include "ptx.cuh"
 #include "tile_copy.cuh"
@@ -165,6 +166,9 @@ __global__ void __launch_bounds__(256, 3)
     const size_t bi = (size_t)x0 + (dir == DY ? (size_t)nx * n_in * o : (size_t)nx * o);
     const size_t bo = (size_t)x0 + (dir == DY ? (size_t)nx * m * o : (size_t)nx * o);
     const int cols = min(W, nx - x0);
+    pdl_trigger();
+    pdl_wait();
+    in = pdl_after(in);
     copy_columns<W>(tile + kHalo * W, in + bi, stride, n_in, cols, vec);
     if (kind != DER)  // the reflected rows: points -4 .. -1 and n_in .. m + 3
         for (int i = t; i < (m - n_in + 2 * kHalo) * W; i += nt) {
@@ -219,6 +223,9 @@ __global__ void __launch_bounds__(256, 3)
     const int t = threadIdx.x, nt = blockDim.x;
     const long l0 = (long)blockIdx.x * W;
     const int rows = (int)min((long)W, nlines - l0);
+    pdl_trigger();
+    pdl_wait();
+    in = pdl_after(in);
     copy_rows(tile + kHalo, pitch, in + (size_t)l0 * n_in, n_in, n_in, rows, vec);
     if (kind != DER) {
         const int nh = m - n_in + 2 * kHalo;
@@ -306,13 +313,15 @@ static int launch_wall_t(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, 
         if (dir == DX) {
             auto kern = ls_wall_x<T, W, L>;
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<(unsigned)grid, threads, smem, ctx->stream>>>(in, out, lo, tb, kind, n_in, lines, pitch, refl, C, vec);
-        } else {
-            auto kern = ls_wall_yz<T, W, L>;
-            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            kern<<<(unsigned)grid, threads, smem, ctx->stream>>>(in, out, lo, tb, kind, n_in, o1, o2, dir, refl, C, vec);
+            return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind,
+                                              n_in, lines, pitch, refl, C, vec),
+                              "ls_wall_x launch");
         }
-        return cuda_check(ctx, cudaGetLastError(), "ls_wall launch");
+        auto kern = ls_wall_yz<T, W, L>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind, n_in,
+                                          o1, o2, dir, refl, C, vec),
+                          "ls_wall_yz launch");
     };
     int rc = run(std::integral_constant<int, 32>{});
     if (rc == X3D_EUNSUPPORTED) rc = run(std::integral_constant<int, 16>{});

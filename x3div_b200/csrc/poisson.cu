@@ -20,6 +20,8 @@
 #include <cmath>
 #include <vector>
 
+#include "launch_pdl.h"
+#include "ptx.cuh"
 #include "x3d_internal.h"
 
 namespace x3d {
@@ -389,12 +391,15 @@ __global__ void __launch_bounds__(kZftThreads, 2)
     zl.ntot = ntot;
     zl.xtab = xtab;
     zl.ztab = tws + N;
+    pdl_trigger();
     for (int t = threadIdx.x; t < 2 * N; t += kZftThreads) tws[t] = __ldg(tw + t);
     if (threadIdx.x < W) {  // ig0 + i0: global index of the tile's first lane
         const int i = min(ig0 + i0 + (int)threadIdx.x, nxh - 1);
         xtab[threadIdx.x] = make_double2(__ldg(tx + i), __ldg(k2x + i));
     }
     __syncthreads();
+    pdl_wait();  // the tables above are the context's own, made before any launch
+    zl.base = pdl_after(zl.base);
     zft<N, W, false, true, kZftThreads, 0, 1, -1, MIR>(zbuf, tws, zl);  // and the inverse, from its fused first stage
 }
 
@@ -519,6 +524,9 @@ __global__ void __launch_bounds__(kXftThreads<M>, 1024 / kXftThreads<M>)
     zl.lstride = P;
     zl.lines = min(W, ny - j0);
     double2 *const out = spec + (size_t)kz * (M + 1) * ny + j0;
+    pdl_trigger();
+    pdl_wait();
+    zl.base = pdl_after(zl.base);
     if constexpr (kXftPaired<M>) {
         constexpr RadixSeq seq = radix_seq(M);
         constexpr int R = kXftLastR<M>, NSL = M / R;
@@ -574,7 +582,9 @@ __global__ void __launch_bounds__(kXftThreads<M>, 1024 / kXftThreads<M>)
     const int kz = blockIdx.x / tiles_j;
     const int j0 = (blockIdx.x - kz * tiles_j) * W;
     const int lines = min(W, ny - j0);
-    const double2 *const in = spec + (size_t)kz * (M + 1) * ny + j0;
+    pdl_trigger();
+    pdl_wait();
+    const double2 *const in = pdl_after(spec) + (size_t)kz * (M + 1) * ny + j0;
     ZLines zl;
     constexpr int P = MIR ? M / 2 : M;  // complex points of a row
     zl.base = reinterpret_cast<double2 *>(f) + ((size_t)kz * ny + j0) * P;
@@ -681,6 +691,9 @@ __global__ void __launch_bounds__(kXftThreads<N>, 1024 / kXftThreads<N>)
     zl.zstride = 1;
     zl.lstride = N;
     zl.lines = (int)min((long)W, nlines - l0);
+    pdl_trigger();
+    pdl_wait();
+    zl.base = pdl_after(zl.base);
     zft<N, W, false, false, kXftThreads<N>, 0, 1, -1, 3>(zbuf, wt, zl);
     for (int i = threadIdx.x; i < W * N; i += kXftThreads<N>) {
         const int l = i % W, k = i / W;  // rows in turn: the shared-memory reads do not conflict
@@ -706,6 +719,9 @@ __global__ void __launch_bounds__(kXftThreads<N>, 1024 / kXftThreads<N>)
     zl.zstride = 1;
     zl.lstride = N;
     zl.lines = (int)min((long)W, nlines - l0);
+    pdl_trigger();
+    pdl_wait();
+    zl.base = pdl_after(zl.base);
     for (int i = threadIdx.x; i < W * N; i += kXftThreads<N>) {
         const int l = i / N, k = i % N;  // along a line, both its reads consecutive
         const double2 z = make_double2(0.0, 0.0);
@@ -856,8 +872,9 @@ static int launch_poisson_z(x3d_ctx_s *ctx, double2 *spec, int nxl, int i0, int 
         const size_t smem = ((size_t)ctx->nz * W + 2 * (size_t)ctx->nz + W) * sizeof(double2);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        kern<<<grid, NT, smem, ctx->stream>>>(spec, nxl, ny_loc, i0, j0, lane_end, ztw, lk2, lt, rk2, rt, ntot);
-        return cuda_check(ctx, cudaGetLastError(), "k_poisson_z");
+        return cuda_check(ctx, launch_pdl(kern, grid, NT, smem, ctx->stream, spec, nxl, ny_loc, i0, j0, lane_end, ztw,
+                                          lk2, lt, rk2, rt, ntot),
+                          "k_poisson_z");
     };
     switch (ctx->nz) {
 #define X3D_ZFT_LAUNCH(N) \
@@ -882,12 +899,11 @@ static int launch_xft(x3d_ctx_s *ctx, double *f, double2 *spec, int ny, int nz, 
         ++ctx->launches;
         if (forward) {
             cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            fwd<<<grid, NT, smem, ctx->stream>>>(f, spec, ny, tw);
+            return cuda_check(ctx, launch_pdl(fwd, grid, NT, smem, ctx->stream, f, spec, ny, tw), "k_rfft_x");
         } else {
             cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            inv<<<grid, NT, smem, ctx->stream>>>(spec, f, ny, tw);
+            return cuda_check(ctx, launch_pdl(inv, grid, NT, smem, ctx->stream, spec, f, ny, tw), "k_irfft_x");
         }
-        return cuda_check(ctx, cudaGetLastError(), forward ? "k_rfft_x" : "k_irfft_x");
     };
     switch (ctx->nx / 2) {
 #define X3D_XFT_LAUNCH(N) \
@@ -907,8 +923,9 @@ static int launch_dct_y(x3d_ctx_s *ctx, int n, double2 *spec, long nlines, const
         const size_t smem = (size_t)n * kXftW * sizeof(double2);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        kern<<<(unsigned)((nlines + kXftW - 1) / kXftW), NT, smem, ctx->stream>>>(spec, nlines, tw);
-        return cuda_check(ctx, cudaGetLastError(), "k_dct_y");
+        return cuda_check(ctx, launch_pdl(kern, (unsigned)((nlines + kXftW - 1) / kXftW), NT, smem, ctx->stream, spec,
+                                          nlines, tw),
+                          "k_dct_y");
     };
     switch (n) {
 #define X3D_YFT_LAUNCH(N) \

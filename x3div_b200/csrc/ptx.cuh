@@ -142,6 +142,20 @@ __device__ __forceinline__ void cp_async(void *dst, const void *src)
 
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
+// The two ends of a programmatic dependent launch (launch_pdl.h): no-ops in a
+// plain launch.  Pointers whose loads the compiler may treat as invariant
+// (const __restrict__ parameters) go through pdl_after, which hides them from
+// it until after the wait, so that no such load moves above it.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename P>
+__device__ __forceinline__ P *pdl_after(P *p)
+{
+    uint64_t v = reinterpret_cast<uint64_t>(p);
+    asm volatile("" : "+l"(v)::"memory");
+    return reinterpret_cast<P *>(v);
+}
+
 // Make generic-proxy writes to shared memory visible to the async proxy.
 __device__ __forceinline__ void fence_proxy_async_smem()
 {
