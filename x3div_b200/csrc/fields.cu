@@ -174,7 +174,7 @@ __global__ void k_scale_y(T *t, const double *ppy, int nx, int ny, size_t n)
     do {                                                                                                    \
         const int bs_ = 256;                                                                                \
         ++ctx->launches;                                                                                    \
-        return cuda_check(ctx, launch_pdl(kern, grid_for(ctx, (n), bs_), bs_, 0, ctx->stream, __VA_ARGS__), \
+        return cuda_check(ctx, launch_pdl(kern, (long)((n) / bs_), grid_for(ctx, (n), bs_), bs_, 0, ctx->stream, __VA_ARGS__), \
                           #kern);                                                                           \
     } while (0)
 

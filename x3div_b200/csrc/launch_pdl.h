@@ -6,7 +6,11 @@
 // before it touches anything another kernel writes or reads; chains of them
 // stay ordered because each waits for the one before.  Between two launches of
 // a few microseconds the launch itself is a third of the time (the 64^3 FP64
-// step, some twenty launches: AAA us with plain launches, BBB so).
+// step, some twenty launches: 147 us with plain launches, 128 so).
+//
+// Launches of kPdlTiles tiles or more are plain: there the start is nothing, and
+// CTAs of the next kernel that sit in the slots of the last ones cost about a
+// hundredth (the 512^3 FP32 sweep 2277 us plain, 2301 so).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -15,8 +19,11 @@
 
 namespace x3d {
 
+constexpr long kPdlTiles = 8192;
+
+// tiles: the tiles of the launch's work, its CTAs unless it is persistent.
 template <typename... P, typename... A>
-inline cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
+inline cudaError_t launch_pdl(void (*kern)(P...), long tiles, unsigned grid, unsigned block, size_t smem, cudaStream_t stream,
                               A &&...args)
 {
     cudaLaunchAttribute attr{};
@@ -28,7 +35,7 @@ inline cudaError_t launch_pdl(void (*kern)(P...), unsigned grid, unsigned block,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = tiles < kPdlTiles ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
 }
 

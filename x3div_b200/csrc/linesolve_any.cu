@@ -268,7 +268,7 @@ int launch_stage_any(x3d_ctx_s *ctx, const StageProgram<T> &prog, bool acc, int 
         if (smem + 1024 > ctx->smem_optin || grid > 0x7fffffffL) return (int)X3D_EUNSUPPORTED;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, prog, args...),
+        return cuda_check(ctx, launch_pdl(kern, grid, (unsigned)grid, threads, smem, ctx->stream, prog, args...),
                           "ls_any launch");
     };
     if (dir == DX) {

@@ -749,7 +749,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                 if (rc) return rc;
             }
             ++ctx->launches;
-            return cuda_check(ctx, launch_pdl(kern, grid, threads, smem, st, prog, nlines, pitch, tile, ntiles,
+            return cuda_check(ctx, launch_pdl(kern, ntiles, grid, threads, smem, st, prog, nlines, pitch, tile, ntiles,
                                               ctx->d_claim, ctx->d_err),
                               "ls_stage_x launch");
         }
@@ -811,7 +811,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
             if (rc) return rc;
         }
         ++ctx->launches;
-        return cuda_check(ctx, launch_pdl(kern, grid, threads, smem, st, maps, prog, nx, ny, dir, box_n, nb, tma_halo,
+        return cuda_check(ctx, launch_pdl(kern, ntiles, grid, threads, smem, st, maps, prog, nx, ny, dir, box_n, nb, tma_halo,
                                           tile, ntiles, ctx->d_claim, ctx->d_err),
                           "ls_stage_yz launch");
 

@@ -313,13 +313,13 @@ static int launch_wall_t(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, 
         if (dir == DX) {
             auto kern = ls_wall_x<T, W, L>;
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind,
+            return cuda_check(ctx, launch_pdl(kern, grid, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind,
                                               n_in, lines, pitch, refl, C, vec),
                               "ls_wall_x launch");
         }
         auto kern = ls_wall_yz<T, W, L>;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return cuda_check(ctx, launch_pdl(kern, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind, n_in,
+        return cuda_check(ctx, launch_pdl(kern, grid, (unsigned)grid, threads, smem, ctx->stream, in, out, lo, tb, kind, n_in,
                                           o1, o2, dir, refl, C, vec),
                           "ls_wall_yz launch");
     };

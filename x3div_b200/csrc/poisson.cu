@@ -872,7 +872,7 @@ static int launch_poisson_z(x3d_ctx_s *ctx, double2 *spec, int nxl, int i0, int 
         const size_t smem = ((size_t)ctx->nz * W + 2 * (size_t)ctx->nz + W) * sizeof(double2);
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        return cuda_check(ctx, launch_pdl(kern, grid, NT, smem, ctx->stream, spec, nxl, ny_loc, i0, j0, lane_end, ztw,
+        return cuda_check(ctx, launch_pdl(kern, grid, grid, NT, smem, ctx->stream, spec, nxl, ny_loc, i0, j0, lane_end, ztw,
                                           lk2, lt, rk2, rt, ntot),
                           "k_poisson_z");
     };
@@ -899,10 +899,10 @@ static int launch_xft(x3d_ctx_s *ctx, double *f, double2 *spec, int ny, int nz, 
         ++ctx->launches;
         if (forward) {
             cudaFuncSetAttribute(fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            return cuda_check(ctx, launch_pdl(fwd, grid, NT, smem, ctx->stream, f, spec, ny, tw), "k_rfft_x");
+            return cuda_check(ctx, launch_pdl(fwd, grid, grid, NT, smem, ctx->stream, f, spec, ny, tw), "k_rfft_x");
         } else {
             cudaFuncSetAttribute(inv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            return cuda_check(ctx, launch_pdl(inv, grid, NT, smem, ctx->stream, spec, f, ny, tw), "k_irfft_x");
+            return cuda_check(ctx, launch_pdl(inv, grid, grid, NT, smem, ctx->stream, spec, f, ny, tw), "k_irfft_x");
         }
     };
     switch (ctx->nx / 2) {
@@ -921,9 +921,10 @@ static int launch_dct_y(x3d_ctx_s *ctx, int n, double2 *spec, long nlines, const
 {
     auto go = [&](auto kern, int NT) {
         const size_t smem = (size_t)n * kXftW * sizeof(double2);
+        const long grid = (nlines + kXftW - 1) / kXftW;
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         ++ctx->launches;
-        return cuda_check(ctx, launch_pdl(kern, (unsigned)((nlines + kXftW - 1) / kXftW), NT, smem, ctx->stream, spec,
+        return cuda_check(ctx, launch_pdl(kern, grid, (unsigned)grid, NT, smem, ctx->stream, spec,
                                           nlines, tw),
                           "k_dct_y");
     };
