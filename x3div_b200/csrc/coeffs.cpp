@@ -323,7 +323,9 @@ void finish_op(OpHost &op)
 // -fw from i to the chunk's end.  Entries past the line's end are zero.
 // Returns the scan depth for thr, or -1 where a factor is not finite or a
 // multiplier above 1 would let a carry grow (no operator of the library).
-static int build_wall_tables(const OpHost &h, int L, double thr, std::vector<double> &tab)
+// uniform: the longest run of whole chunks whose s, w and fw each stay within
+// eps (relative; under the rounding of the type) of their first entry.
+static int build_wall_tables(const OpHost &h, int L, double thr, double eps, std::vector<double> &tab, int uniform[2])
 {
     const int n = h.n, C = (n + L - 1) / L, P = C * L;
     tab.assign((size_t)5 * P + 2 * C, 0.0);
@@ -375,8 +377,8 @@ int upload_op(x3d_op_s *op)
     std::vector<double> wall[2];
     bool walls = !h.periodic;
     if (walls) {
-        op->wall_depth[0] = build_wall_tables(h, kChunkLong<float>, 1e-12, wall[0]);
-        op->wall_depth[1] = build_wall_tables(h, kChunkLong<double>, 1e-20, wall[1]);
+        op->wall_depth[0] = build_wall_tables(h, kChunkLong<float>, 1e-12, 1e-9, wall[0], op->wall_uniform[0]);
+        op->wall_depth[1] = build_wall_tables(h, kChunkLong<double>, 1e-20, 4e-16, wall[1], op->wall_uniform[1]);
         walls = op->wall_depth[0] > 0 && op->wall_depth[1] > 0;
     }
     const size_t o_wf = al(o_d + 5 * n * sizeof(double));

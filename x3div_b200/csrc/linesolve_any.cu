@@ -248,7 +248,8 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
 
 // The derivative sweep (18 operators of one field, three launches) took 1547 us
 // at 171 x 129 x 150 FP64 on ls_generic and takes 182 us here (2.8 TB/s of one
-// read per direction and the outputs); 1575 and 199 us at 250 x 171 x 129 FP32.
+// read per direction and the outputs; 170 with the shifted twins); 1575 and 155
+// us at 250 x 171 x 129 FP32.
 // prog: its responses filled for chunks of kChunkLong<T> points (launch_stage
 // did), acc: it needs the accumulator or a general flush.
 template <typename T, int W>
@@ -294,6 +295,7 @@ int launch_stage_any(x3d_ctx_s *ctx, const StageProgram<T> &prog, bool acc, int 
     return launch(ls_any_yz<T, W, L, false, 1>, smem, grid, nx, ny, dir, C, tile);
 }
 
+template int launch_stage_any<float, 32>(x3d_ctx_s *, const StageProgram<float> &, bool, int, int, int, int);
 template int launch_stage_any<float, 16>(x3d_ctx_s *, const StageProgram<float> &, bool, int, int, int, int);
 template int launch_stage_any<float, 8>(x3d_ctx_s *, const StageProgram<float> &, bool, int, int, int, int);
 template int launch_stage_any<double, 16>(x3d_ctx_s *, const StageProgram<double> &, bool, int, int, int, int);

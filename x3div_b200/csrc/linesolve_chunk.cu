@@ -708,6 +708,16 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
             if constexpr (PR == 1 && OCC == 1 && !PERSIST && L == kChunkLong<T> && W <= 16)
                 if (!prog.aligned_only) {
                     fill_resp(prog, L, n);
+                    // FP32: 32 lines a tile where plain programs still fit 256
+                    // threads.  A warp then holds one chunk of 32 lines, so a
+                    // short last chunk does not run beside a full one in the
+                    // same warp (250 x 171 x 129 sweep 189 -> 155 us; FP64
+                    // lines of that length do not fit)
+                    if constexpr (W == 16 && sizeof(T) == 4)
+                        if (!acc && C * 32 <= 256) {
+                            const int rc = launch_stage_any<T, 32>(ctx, prog, acc, dir, nx, ny, nz);
+                            if (rc != X3D_EUNSUPPORTED) return rc;
+                        }
                     return launch_stage_any<T, W>(ctx, prog, acc, dir, nx, ny, nz);
                 }
             return X3D_EUNSUPPORTED;

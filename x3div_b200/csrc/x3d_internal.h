@@ -86,10 +86,11 @@ struct x3d_op_s {
     bool builtin = false;
     // Non-periodic operators: the chunked solve's tables (linesolve_walls.cu),
     // inside dmem; null where the factors do not bound the sweeps.  wall_depth:
-    // chunks a carry scan visits, FP32 and FP64.
+    // chunks a carry scan visits, FP32 and FP64
     const float *wallf = nullptr;
     const double *walld = nullptr;
     int wall_depth[2] = {0, 0};
+    int wall_uniform[2][2] = {};  // first and last + 1 chunk whose factors are one value each
 };
 
 struct x3d_ctx_s {
