@@ -79,3 +79,49 @@ def test_batch_sweep(oracle, torch_cuda, prec, tuned):
                 ref = oracle.apply(kind, d, used, 2 * np.pi / b[d])
                 assert rel_err(to_host(os_[0][d][k]), ref) < tol, (b, d, kind)
     batch.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("tuned", [False, True])
+def test_batch_jobs_of_one_shape_with_different_twins(oracle, torch_cuda, prec, tuned):
+    """Every other field sends the families its caller does not want (derpv
+    and interpv) to one dump array per job, so that only the others' solves
+    have shifted outputs: jobs of one box shape and direction then differ in
+    the operators they solve, and a CTA goes from one kind to the other many
+    times over the 24 fields."""
+    torch = torch_cuda
+    from x3div_b200 import Batch, to_device, to_host
+    boxes = [(48, 32, 40), (32, 24, 16)]
+    nfields = 24
+    dt = torch.float64 if prec == "f64" else torch.float32
+    fields = [[to_device(seeded_field(b, seed=100 * i + f, noise=1e-2), dt) for f in range(nfields)]
+              for i, b in enumerate(boxes)]
+    outs = []
+    for fs in fields:
+        per_field = []
+        for f, u in enumerate(fs):
+            per_dir = []
+            for _ in range(3):
+                row = [torch.full_like(u, float("nan")) for _ in range(6)]
+                if f % 2:
+                    row[5] = row[3]
+                per_dir.append(row)
+            per_field.append(per_dir)
+        outs.append(per_field)
+    batch = Batch(boxes, precision=prec)
+    batch.bind_sweep(fields, outs)
+    if tuned:
+        batch.autotune()
+    batch.run()
+    batch.sync()
+    tol = 1e-12 if prec == "f64" else 1e-5
+    for b, fs, os_ in zip(boxes, fields, outs):
+        for f, u in enumerate(fs):
+            used = to_host(u).astype(np.float64)
+            for d in range(3):
+                for k, kind in enumerate(("der", "der2", "dervp", "derpv", "intvp", "intpv")):
+                    if f % 2 and k in (3, 5):
+                        continue
+                    ref = oracle.apply(kind, d, used, 2 * np.pi / b[d])
+                    assert rel_err(to_host(os_[f][d][k]), ref) < tol, (b, f, d, kind)
+    batch.close()

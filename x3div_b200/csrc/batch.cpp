@@ -137,6 +137,7 @@ int make_jobs(x3d_batch_s *b, std::vector<BatchJob<T>> &jobs, size_t *tile_cap_o
                 }
                 // the shifted twins: derpv and interpv as second outputs of
                 // dervp and intervp, where x rows can be stored as vectors
+                int merged = 0;  // bit k: family k is another's second output
                 for (int k = 0, kept = 0, n0 = J.nops; k < n0; ++k) {
                     int vp = -1;
                     bool twice = false;  // the order of writes to one output stays as listed
@@ -148,6 +149,7 @@ int make_jobs(x3d_batch_s *b, std::vector<BatchJob<T>> &jobs, size_t *tile_cap_o
                     if (vp >= 0) {
                         J.shift_out[vp] = J.out[k];
                         --J.nops;
+                        merged |= 1 << k;
                     } else {
                         J.op[kept] = J.op[k];
                         J.kind[kept] = J.kind[k];
@@ -162,8 +164,9 @@ int make_jobs(x3d_batch_s *b, std::vector<BatchJob<T>> &jobs, size_t *tile_cap_o
                 const int xs = L_force > 0 ? x_force : b->choice_X[sd];
                 size_t tb = 0;
                 if (plan_batch_job<T>(J, L, w, xs, &tb)) {
-                    // one box shape's operators along d at one chunk length
-                    J.rclass = sd * 2 + (J.L == kChunkLong<T> ? 0 : 1);
+                    // one box shape's operators along d at one chunk length,
+                    // but for the merged ones, which depend on the job's outputs
+                    J.rclass = (sd * 2 + (J.L == kChunkLong<T> ? 0 : 1)) * 64 + merged;
                     J.tile0 = tiles;
                     tiles += J.ntiles;
                     tile_cap = std::max(tile_cap, tb);
