@@ -106,3 +106,46 @@ def test_batch_autotune_keeps_results(oracle, torch_cuda, prec):
     batch.sync()
     check()
     batch.close()
+
+
+@pytest.mark.parametrize("prec", ["f32", "f64"])
+@pytest.mark.parametrize("tuned", [False, True])
+def test_batch_with_unaligned_arrays(oracle, torch_cuda, prec, tuned):
+    """Inputs and outputs one element into their allocations, alone and
+    together: x jobs store 16-byte vectors, so any unaligned array of one
+    sends it to the fallback launches; y and z jobs store single elements and
+    keep unaligned outputs."""
+    torch = torch_cuda
+    from x3div_b200 import Batch, to_device, to_host
+    dt = torch.float32 if prec == "f32" else torch.float64
+    tol = 1e-5 if prec == "f32" else 1e-12
+    boxes = [(32, 24, 16), (64, 40, 24)]
+
+    def shifted(like, off):
+        return torch.full((like.numel() + off,), np.nan, dtype=dt, device="cuda")[off:].view(like.shape)
+
+    # per field: offset of the input, and of each of the six outputs
+    layouts = [(0, (0, 0, 0, 0, 0, 0)), (0, (1, 0, 0, 0, 0, 0)), (0, (0, 0, 0, 1, 0, 0)), (0, (1, 1, 1, 1, 1, 1)),
+               (1, (0, 0, 0, 0, 0, 0))]
+    fields, outs = [], []
+    for i, b in enumerate(boxes):
+        base = [to_device(seeded_field(b, 700 + 10 * i + f, noise=1e-2), dt) for f in range(len(layouts))]
+        fields.append([shifted(u, off).copy_(u) for u, (off, _) in zip(base, layouts)])
+        outs.append([[[shifted(u, o) for o in offs] for _ in range(3)] for u, (_, offs) in zip(base, layouts)])
+    batch = Batch(boxes, precision=prec)
+    batch.bind_sweep(fields, outs)
+    # x of the layouts 1 to 3, and every direction of the unaligned input
+    assert batch.info()["fallback_jobs"] == len(boxes) * (3 + 3)
+    if tuned:
+        batch.autotune()
+    batch.run()
+    batch.sync()
+    for i, b in enumerate(boxes):
+        for f, u in enumerate(fields[i]):
+            used = to_host(u).astype(np.float64)
+            for d in range(3):
+                for k, kind in enumerate(KINDS):
+                    ref = oracle.apply(kind, d, used, 2 * np.pi / b[d])
+                    err = rel_err(to_host(outs[i][f][d][k]), ref)
+                    assert err < tol, (b, f, d, kind, err)
+    batch.close()

@@ -1370,11 +1370,11 @@ bool plan_batch_job(BatchJob<T> &J, int L, int w_req, int xstage, size_t *tile_b
     if (W * J.C > kBatchThreads || W > 256) return false;
     J.W = W;
     if (J.dir == DX) {
-        if (n % V || (reinterpret_cast<uintptr_t>(J.in) & 15)) return false;
-        // staged outputs leave as bulk row copies: 16-byte aligned rows
+        // rows move as 16-byte vectors or bulk copies, in and out
+        if (n % V || !al16(J.in)) return false;
+        for (int k = 0; k < J.nops; ++k)
+            if (!al16(J.out[k]) || !al16(J.shift_out[k])) return false;
         J.xstage = xstage ? 1 : 0;
-        for (int k = 0; k < J.nops && J.xstage; ++k)
-            if (reinterpret_cast<uintptr_t>(J.out[k]) & 15) J.xstage = 0;
         int pitch = J.C * L + 2 * kHalo;
         while (((size_t)pitch * es / 16) % 2 == 0) pitch += V;
         J.pitch = pitch;
