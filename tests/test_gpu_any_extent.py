@@ -101,3 +101,44 @@ def test_stages_on_odd_extents(oracle, torch_cuda, shape, prec):
     for got, want in zip(u, uh):
         assert rel_err(to_host(got), want) < max(bound, 1e-11 if prec == "f64" else 1e-4)
     ctx.close()
+
+
+# (32, 112, 256) is an extent whose divergence along z an untuned FP32 context
+# solves in packed pairs (configuration 14), which store the FP64 result two
+# points at a time
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape,cfg", [((32, 112, 256), -1), ((64, 24, 32), 12), ((64, 24, 32), 14),
+                                       ((64, 24, 32), 15), ((64, 24, 32), -1)])
+@pytest.mark.parametrize("off_u,off_p", [(0, 1), (1, 0), (1, 1)])
+def test_stages_on_unaligned_fields(oracle, torch_cuda, shape, cfg, prec, off_u, off_p):
+    """The velocity and its work arrays off_u, the FP64 pressure off_p
+    elements into their allocations."""
+    torch = torch_cuda
+    from x3div_b200 import Context, to_device, to_host
+    ctx = Context(*shape, lengths=LEN, precision=prec)
+    ctx.set_kernel(cfg)
+    dt_ = torch.float64 if prec == "f64" else torch.float32
+    tol = 1e-12 if prec == "f64" else 1e-4
+
+    def new(dtype, off):
+        n = shape[0] * shape[1] * shape[2]
+        return torch.full((n + off,), float("nan"), dtype=dtype, device="cuda")[off:].view(shape[::-1])
+
+    u = [new(dt_, off_u).copy_(to_device(seeded_field(shape, s, lengths=LEN, noise=1e-2), dt_)) for s in (1, 2, 3)]
+    uh = [to_host(a).astype(np.float64) for a in u]
+    h = (ctx.dx, ctx.dy, ctx.dz)
+    p = new(torch.float64, off_p)
+    g, du = ([new(dt_, off_u) for _ in range(3)] for _ in range(2))
+    ctx.divergence(p, *u)
+    ctx.momentum_rhs_eq(*du, *u)
+    ctx.sync()
+    assert rel_err(to_host(p), oracle.divergence(*uh, *h)) < tol
+    for got, want in zip(du, oracle.momentum_rhs(*uh, *h)):
+        assert rel_err(to_host(got), want) < tol
+    ph = seeded_field(shape, 30, kind="rand", lengths=LEN, noise=0)
+    p.copy_(to_device(ph))
+    ctx.gradp(*g, p)
+    ctx.sync()
+    for got, want in zip(g, oracle.gradp(ph, *h)):
+        assert rel_err(to_host(got), want) < tol
+    ctx.close()

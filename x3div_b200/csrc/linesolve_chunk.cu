@@ -726,12 +726,14 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         if (OCC > 1 && (acc || threads > 256)) return X3D_EUNSUPPORTED;
         cudaStream_t st = ctx->stream;
         if constexpr (PR == 2) {
-            // paired y/z lines: even x extent, 8-byte aligned pair stores
+            // paired y/z lines: even x extent; pairs are loaded and stored whole,
+            // 8 bytes of FP32 or 16 of FP64
             if (dir == DX || nx % 2) return X3D_EUNSUPPORTED;
             for (int k = 0; k < prog.nops; ++k) {
                 const StageOp<T> &so = prog.ops[k];
-                if (so.flush &&
-                    (!al8(so.out) || !al8(so.base) || !al8(so.out2) || !al8(so.base2) || !al8(so.shift_out)))
+                auto pairs = [&](const void *p) { return so.out_f64 ? al16(p) : al8(p); };
+                if (so.flush && (!pairs(so.out) || !pairs(so.base) || !pairs(so.out2) || !pairs(so.base2) ||
+                                 !al8(so.shift_out)))
                     return X3D_EUNSUPPORTED;
             }
         } else if (dir == DX) {
