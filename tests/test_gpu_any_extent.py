@@ -142,3 +142,54 @@ def test_stages_on_unaligned_fields(oracle, torch_cuda, shape, cfg, prec, off_u,
     for got, want in zip(g, oracle.gradp(ph, *h)):
         assert rel_err(to_host(got), want) < tol
     ctx.close()
+
+
+# an extent of own x transforms, one of cuFFT's (x, y) plane and fused z
+# transforms, and one of its 3-D transform
+@pytest.mark.parametrize("shape", [(32, 20, 16), (20, 12, 24), (18, 12, 10)])
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+def test_pressure_one_element_into_its_allocation(oracle, torch_cuda, shape, prec):
+    """The periodic solve alone, inside a step and inside a captured step."""
+    torch = torch_cuda
+    from x3div_b200 import Context, X3DError, to_device, to_host
+    stream = torch.cuda.Stream()
+    ctx = Context(*shape, lengths=LEN, precision=prec, stream=stream)
+    dt_ = torch.float64 if prec == "f64" else torch.float32
+    n = shape[0] * shape[1] * shape[2]
+
+    def new(off):
+        return torch.full((n + off,), float("nan"), dtype=torch.float64, device="cuda")[off:].view(shape[::-1])
+
+    rhs = seeded_field(shape, 21, kind="rand", lengths=LEN, noise=0)
+    p = new(1).copy_(to_device(rhs))
+    torch.cuda.synchronize()
+    ctx.poisson(p)
+    ctx.sync()
+    assert rel_err(to_host(p), oracle.poisson(rhs, *LEN)) < 1e-12
+    u0 = [to_device(seeded_field(shape, s, lengths=LEN, noise=1e-2), dt_) for s in (1, 2, 3)]
+    uh = [to_host(a).astype(np.float64) for a in u0]
+    bound = 99 * 2 / min(ctx.dx, ctx.dy, ctx.dz) * max(LEN) / (2 * np.pi) * (2.0**-53 if prec == "f64" else 2.0**-24)
+
+    def state():
+        u = [a.clone() for a in u0]
+        return u, [torch.empty_like(a) for a in u], new(1), [torch.empty_like(a) for a in u]
+
+    eager, captured = state(), state()
+    torch.cuda.synchronize()
+    u, du, q, g = eager
+    ctx.euler_step(*u, *du, q, *g, 1e-3)
+    ctx.close()
+    ctx = Context(*shape, lengths=LEN, precision=prec, stream=stream)  # nothing allocated yet
+    u, du, q, g = captured
+    ctx.step_capture(*u, *du, q, *g, 1e-3)
+    ctx.step_launch()
+    ctx.sync()
+    assert torch.equal(eager[2], captured[2])
+    for a, b in zip(eager[0] + eager[3], captured[0] + captured[3]):
+        assert torch.equal(a, b)
+    oracle.euler_step(*uh, 1e-3, lengths=LEN)
+    for a, want in zip(u, uh):  # the bound of test_stages_on_odd_extents
+        assert rel_err(to_host(a), want) < max(bound, 1e-11 if prec == "f64" else 1e-4)
+    with pytest.raises(X3DError):  # a complex array has no such address
+        ctx.poisson_zpencil(new(1), 1, 0, 1, 0)
+    ctx.close()

@@ -904,7 +904,8 @@ int x3d_poisson_zpencil(x3d_ctx ctx, void *spec, int nxh_loc, int i0, int ny_loc
     int rc = check_ctx(ctx);
     if (rc) return rc;
     if ((rc = need_periodic(ctx))) return rc;
-    if (!spec || !is_device_ptr(spec)) return set_error(ctx, X3D_EINVAL, "spec must be a device array");
+    if (!spec || !is_device_ptr(spec) || reinterpret_cast<uintptr_t>(spec) % 16)
+        return set_error(ctx, X3D_EINVAL, "spec must be a device array of complex values, 16-byte aligned");
     return poisson_zpencil(ctx, spec, nxh_loc, i0, ny_loc, j0);
 }
 
@@ -1256,7 +1257,7 @@ int x3d_step_capture(x3d_ctx ctx, void *ux1, void *uy1, void *uz1, void *dux1, v
     }
     // everything the step allocates on first use, before the capture
     if (!ctx_scratch(ctx, 5)) return set_error(ctx, X3D_ENOMEM, "scratch allocation failed");
-    if ((rc = poisson_setup(ctx))) return rc;
+    if ((rc = poisson_reserve(ctx, static_cast<const double *>(dev[6])))) return rc;
     if ((rc = cuda_check(ctx, cudaStreamSynchronize(ctx->stream), "capture"))) return rc;
     if (ctx->step_exec) cudaGraphExecDestroy(ctx->step_exec);
     if (ctx->step_graph) cudaGraphDestroy(ctx->step_graph);

@@ -953,11 +953,30 @@ static int launch_divide(x3d_ctx_s *ctx, double2 *c, int nxl, int nyl, size_t n,
     return cuda_check(ctx, cudaGetLastError(), "k_spectral_divide");
 }
 
+// What a solve of rhs allocates on first use.
+int poisson_reserve(x3d_ctx_s *ctx, const double *rhs)
+{
+    const int rc = poisson_setup(ctx);
+    if (rc || reinterpret_cast<uintptr_t>(rhs) % 16 == 0 || ctx->aligned_rhs) return rc;
+    if (cudaMalloc(&ctx->aligned_rhs, ctx->npts() * sizeof(double)) != cudaSuccess) {
+        ctx->aligned_rhs = nullptr;
+        return set_error(ctx, X3D_ENOMEM, "aligned right-hand side allocation failed");
+    }
+    return X3D_OK;
+}
+
 int poisson_solve(x3d_ctx_s *ctx, double *rhs)
 {
     const TraceRange trace("poisson");
-    int rc = poisson_setup(ctx);
+    int rc = poisson_reserve(ctx, rhs);
     if (rc) return rc;
+    if (reinterpret_cast<uintptr_t>(rhs) % 16) {
+        // pairs of reals are moved as 16-byte units (cuFFT asks for as much)
+        const size_t bytes = ctx->npts() * sizeof(double);
+        rc = launch_copy(ctx, ctx->aligned_rhs, rhs, bytes);
+        rc = rc ? rc : poisson_solve(ctx, ctx->aligned_rhs);
+        return rc ? rc : launch_copy(ctx, rhs, ctx->aligned_rhs, bytes);
+    }
     if (poisson_own_x(ctx)) {
         // x transforms (spectrum y fastest), y transforms, z solve, and back
         auto *spec = static_cast<double2 *>(ctx->spectrum);
@@ -1196,6 +1215,8 @@ void poisson_free(x3d_ctx_s *ctx)
     ctx->plans_ready = false;
     if (ctx->spectrum) cudaFree(ctx->spectrum);
     ctx->spectrum = nullptr;
+    if (ctx->aligned_rhs) cudaFree(ctx->aligned_rhs);
+    ctx->aligned_rhs = nullptr;
     if (ctx->d_k2x) cudaFree(ctx->d_k2x);
     ctx->d_k2x = nullptr;
     if (ctx->d_zft_tw) cudaFree(ctx->d_zft_tw);

@@ -143,6 +143,8 @@ struct x3d_ctx_s {
     // its walls, and the mirrored right-hand side (created on first use)
     x3d_ctx_s *mirror = nullptr;
     double *mirror_rhs = nullptr;
+    // copy of a right-hand side off a 16-byte boundary (created on first use)
+    double *aligned_rhs = nullptr;
     double *d_k2x = nullptr, *d_tx = nullptr, *d_k2y = nullptr, *d_ty = nullptr, *d_k2z = nullptr,
            *d_tz = nullptr;
     // scratch fields owned by the context (sized nx*ny*nz elements)
@@ -269,6 +271,7 @@ int reduce_absmax_mean(x3d_ctx_s *ctx, const double *p, size_t n, double *out);
 
 // ---- Poisson (poisson.cu) ------------------------------------------------
 int poisson_setup(x3d_ctx_s *ctx);
+int poisson_reserve(x3d_ctx_s *ctx, const double *rhs);
 int poisson_solve(x3d_ctx_s *ctx, double *rhs);
 // the solve with homogeneous Neumann conditions along the non-periodic
 // directions, rhs on the pressure grid (ppts points)
