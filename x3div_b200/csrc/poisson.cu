@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "launch_pdl.h"
+#include "poisson_tables.h"
 #include "ptx.cuh"
 #include "x3d_internal.h"
 
@@ -31,8 +32,10 @@ namespace x3d {
 //   k2[i] = (n wp / L)^2, wp = (acix6 2 d sin(w/2) + bcix6 2 d sin(3w/2)) / (1 + 2 alcaix6 cos w)
 //   t[i]  = (2 aicix6 cos(r/2) + 2 (bicix6 cos(1.5r) + cicix6 cos(2.5r) + dicix6 cos(3.5r)))
 //           / (1 + 2 ailcaix6 cos r),  r = exs(i) d
-static void waves_tables(int n, double len, std::vector<double> &k2, std::vector<double> &t)
+static WaveTables waves_tables(int n, double len)
 {
+    WaveTables out;
+    std::vector<double> &k2 = out.k2, &t = out.t;
     const double twopi = 2.0 * std::acos(-1.0);
     const double d = len / n;
     double alcai, aci, bci, c_, d_;
@@ -61,6 +64,7 @@ static void waves_tables(int n, double len, std::vector<double> &k2, std::vector
         const double t1 = 1.0 + 2.0 * ailcai * std::cos(r);
         t[i] = (tt1 + tt) / t1;
     }
+    return out;
 }
 
 // c(i,j,k) <- -c / (K ntot), K = k2x Ty^2 Tz^2 + k2y Tx^2 Tz^2 + k2z Tx^2 Ty^2
@@ -403,18 +407,6 @@ __global__ void __launch_bounds__(kZftThreads, 2)
     zft<N, W, false, true, kZftThreads, 0, 1, -1, MIR>(zbuf, tws, zl);  // and the inverse, from its fused first stage
 }
 
-// The z lengths with a fused kernel.
-#define X3D_ZFT_SIZES(X) X(8) X(12) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256) X(384) X(512) X(768) X(1024)
-
-static bool zft_supported(int n)
-{
-#define X3D_ZFT_CASE(N) \
-    if (n == N) return true;
-    X3D_ZFT_SIZES(X3D_ZFT_CASE)
-#undef X3D_ZFT_CASE
-    return false;
-}
-
 // ---------------------------------------------------------------------------
 // Own x transforms: a real line of n = 2M points as the complex line z[m] =
 // f[2m] + i f[2m+1] of M points (the same memory), transformed by the
@@ -733,78 +725,48 @@ __global__ void __launch_bounds__(kXftThreads<N>, 1024 / kXftThreads<N>)
     zft<N, W, true, false, kXftThreads<N>, 0, 1, -1, 3>(zbuf, wt, zl);
 }
 
-// The 1-D modified-wavenumber tables and, where a fused z kernel exists for
-// nz, its twiddles: all that the z part of the solve reads.
+// Device memory of the tables.
+struct TableMem {
+    void *alloc(size_t bytes)
+    {
+        void *p = nullptr;
+        return cudaMalloc(&p, bytes) == cudaSuccess ? p : nullptr;
+    }
+    bool upload(void *dst, const void *src, size_t bytes)
+    {
+        return cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
+    }
+    void release(void *p) { cudaFree(p); }
+};
+
+static int place_tables(x3d_ctx_s *ctx, const std::vector<double> &block, double **out)
+{
+    TableMem mem;
+    switch (place_block(mem, block, out)) {
+    case Placed::no_memory: return set_error(ctx, X3D_ENOMEM, "poisson tables");
+    case Placed::no_upload: return set_error(ctx, X3D_ECUDA, "poisson tables upload");
+    default: return X3D_OK;
+    }
+}
+
+// The 1-D modified-wavenumber tables and the own transforms' twiddles, made on
+// first use.
 static int poisson_tables(x3d_ctx_s *ctx)
 {
     if (ctx->d_k2x) return X3D_OK;
-    const int nx = ctx->nx, ny = ctx->ny, nz = ctx->nz;
-    std::vector<double> k2x, tx, k2y, ty, k2z, tz;
-    waves_tables(nx, ctx->xlx, k2x, tx);
-    waves_tables(ny, ctx->yly, k2y, ty);
-    waves_tables(nz, ctx->zlz, k2z, tz);
-    double *tab = nullptr;
-    const size_t tot = 2 * ((size_t)nx + ny + nz);
-    if (cudaMalloc(&tab, tot * sizeof(double)) != cudaSuccess) return set_error(ctx, X3D_ENOMEM, "poisson tables");
-    std::vector<double> h;
-    h.reserve(tot);
-    h.insert(h.end(), k2x.begin(), k2x.end());
-    h.insert(h.end(), tx.begin(), tx.end());
-    h.insert(h.end(), k2y.begin(), k2y.end());
-    h.insert(h.end(), ty.begin(), ty.end());
-    h.insert(h.end(), k2z.begin(), k2z.end());
-    h.insert(h.end(), tz.begin(), tz.end());
-    if (cudaMemcpy(tab, h.data(), tot * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
-        cudaFree(tab);
-        return set_error(ctx, X3D_ECUDA, "poisson tables upload");
-    }
-    ctx->d_k2x = tab;
-    ctx->d_tx = tab + nx;
-    ctx->d_k2y = tab + 2 * nx;
-    ctx->d_ty = tab + 2 * nx + ny;
-    ctx->d_k2z = tab + 2 * nx + 2 * ny;
-    ctx->d_tz = tab + 2 * nx + 2 * ny + nz;
-    if (zft_supported(nz)) {  // the twiddles, then (tz, k2z) of each z mode
-        std::vector<double> tw(4 * (size_t)nz);
-        const double twopi = 2.0 * std::acos(-1.0);
-        for (int t = 0; t < nz; ++t) {
-            tw[2 * t] = std::cos(twopi * t / nz);
-            tw[2 * t + 1] = -std::sin(twopi * t / nz);
-            tw[2 * ((size_t)nz + t)] = tz[t];
-            tw[2 * ((size_t)nz + t) + 1] = k2z[t];
-        }
-        if (cudaMalloc(&ctx->d_zft_tw, tw.size() * sizeof(double)) != cudaSuccess)
-            return set_error(ctx, X3D_ENOMEM, "poisson twiddles");
-        if (cudaMemcpy(ctx->d_zft_tw, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice) !=
-            cudaSuccess) {
-            cudaFree(ctx->d_zft_tw);
-            ctx->d_zft_tw = nullptr;
-            return set_error(ctx, X3D_ECUDA, "poisson twiddles upload");
-        }
-    }
-    if (nx % 2 == 0 && zft_supported(nx / 2)) {
-        const int m = nx / 2;
-        const double twopi = 2.0 * std::acos(-1.0);
-        std::vector<double> tw(2 * (size_t)(2 * m + 1));
-        for (int t = 0; t < m; ++t) {
-            tw[2 * t] = std::cos(twopi * t / m);
-            tw[2 * t + 1] = -std::sin(twopi * t / m);
-        }
-        for (int k = 0; k <= m; ++k) {
-            tw[2 * (m + k)] = std::cos(twopi * k / nx);
-            tw[2 * (m + k) + 1] = -std::sin(twopi * k / nx);
-        }
-        if (cudaMalloc(&ctx->d_xft_tw, tw.size() * sizeof(double)) != cudaSuccess) {
-            ctx->d_xft_tw = nullptr;
-            return set_error(ctx, X3D_ENOMEM, "poisson x twiddles");
-        }
-        if (cudaMemcpy(ctx->d_xft_tw, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice) !=
-            cudaSuccess) {
-            cudaFree(ctx->d_xft_tw);
-            ctx->d_xft_tw = nullptr;
-            return set_error(ctx, X3D_ECUDA, "poisson x twiddles upload");
-        }
-    }
+    const PoissonTables t = poisson_host_tables(waves_tables(ctx->nx, ctx->xlx), waves_tables(ctx->ny, ctx->yly),
+                                                waves_tables(ctx->nz, ctx->zlz));
+    double *d = nullptr;
+    const int rc = place_tables(ctx, t.block, &d);
+    if (rc) return rc;
+    ctx->d_k2x = d + t.k2x;  // the block itself
+    ctx->d_tx = d + t.tx;
+    ctx->d_k2y = d + t.k2y;
+    ctx->d_ty = d + t.ty;
+    ctx->d_k2z = d + t.k2z;
+    ctx->d_tz = d + t.tz;
+    ctx->d_zft_tw = t.ztw ? d + t.ztw : nullptr;
+    ctx->d_xft_tw = t.xtw ? d + t.xtw : nullptr;
     return X3D_OK;
 }
 
@@ -1123,14 +1085,7 @@ static int poisson_solve_halves(x3d_ctx_s *mc, double *rhs, const int m[3], cons
             tw[2 * (n + t)] = std::cos(pi * t / (2.0 * n));
             tw[2 * (n + t) + 1] = -std::sin(pi * t / (2.0 * n));
         }
-        double *d = nullptr;
-        if (cudaMalloc(&d, tw.size() * sizeof(double)) != cudaSuccess)
-            return set_error(mc, X3D_ENOMEM, "poisson y twiddles");
-        if (cudaMemcpy(d, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) {
-            cudaFree(d);
-            return set_error(mc, X3D_ECUDA, "poisson y twiddles upload");
-        }
-        mc->d_yft_tw = d;
+        if ((rc = place_tables(mc, tw, &mc->d_yft_tw))) return rc;
     }
     if (!half[1] && !mc->plan_yh_ready) {
         int n = mc->ny;
@@ -1217,12 +1172,8 @@ void poisson_free(x3d_ctx_s *ctx)
     ctx->spectrum = nullptr;
     if (ctx->aligned_rhs) cudaFree(ctx->aligned_rhs);
     ctx->aligned_rhs = nullptr;
-    if (ctx->d_k2x) cudaFree(ctx->d_k2x);
-    ctx->d_k2x = nullptr;
-    if (ctx->d_zft_tw) cudaFree(ctx->d_zft_tw);
-    ctx->d_zft_tw = nullptr;
-    if (ctx->d_xft_tw) cudaFree(ctx->d_xft_tw);
-    ctx->d_xft_tw = nullptr;
+    if (ctx->d_k2x) cudaFree(ctx->d_k2x);  // the block of all tables
+    ctx->d_k2x = ctx->d_zft_tw = ctx->d_xft_tw = nullptr;
     if (ctx->d_yft_tw) cudaFree(ctx->d_yft_tw);
     ctx->d_yft_tw = nullptr;
     if (ctx->half_spectrum) cudaFree(ctx->half_spectrum);
