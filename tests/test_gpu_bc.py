@@ -312,3 +312,56 @@ def test_nonperiodic_poisson_on_halves(oracle, torch_cuda, shape, per, offset):
             assert ctx.launch_count() - n0 == (3 if per[1] else 5)
         assert rel_err(to_host(rhs), oracle.poisson_bc(np.asfortranarray(g), lengths, per)) < 1e-12, (shape, per, seed)
     ctx.close()
+
+
+def _walled_y_solution(rhs, lengths):
+    """The solve with walls along y in long double: the modes of poisson_bc
+    with the wavenumbers of waves() (src/poisson.f90:483-703)."""
+    import scipy.fft
+    ld = np.longdouble
+    pi = 4 * np.arctan(ld(1))
+
+    def waves(n, modes, length):
+        d = ld(length) / n
+        i = np.arange(modes).astype(ld)
+        w = 2 * pi * np.minimum(i, n - i) / n
+        wp = (2 * ld(63) / 62 * np.sin(w / 2) + 2 * ld(17) / 186 * np.sin(3 * w / 2)) / (1 + ld(9) / 31 * np.cos(w))
+        al = ld(49) / 100
+        c = ((75 + 70 * al) / 64, (126 * al - 25) / 128, (3 - 10 * al) / 128)
+        t = sum(k * np.cos((j + ld(1) / 2) * w) for j, k in enumerate(c)) / (1 + 2 * al * np.cos(w))
+        return (wp / d)**2, t
+
+    nx, ny, nz = rhs.shape
+    (kx, tx), (ky, ty), (kz, tz) = (waves(n * f, n, le * f) for n, f, le in
+                                    zip((nx, ny, nz), (1, 2, 1), lengths))
+    at = (np.s_[:, None, None], np.s_[None, :, None], np.s_[None, None, :])
+    kx, tx, ky, ty, kz, tz = kx[at[0]], tx[at[0]], ky[at[1]], ty[at[1]], kz[at[2]], tz[at[2]]
+    k = kx * (ty * tz)**2 + ky * (tx * tz)**2 + kz * (tx * ty)**2
+    f = scipy.fft.dct(rhs.astype(ld), type=2, axis=1)
+    f = scipy.fft.fftn(f.astype(np.clongdouble), axes=(0, 2))
+    f = np.where(k < 1e-16, 0, -f / np.maximum(k, ld(1e-16)))
+    f = scipy.fft.ifftn(f, axes=(0, 2)).real
+    return scipy.fft.idct(f, type=2, axis=1)
+
+
+# the longest cosine transforms, in cubic cells: 2-norm errors, means of four
+# fields, measured 6.2e-16, 4.4e-16 and 9.5e-16 (6.7e-16, 6.1e-16 and 10.2e-16
+# with each twiddle the product of the one before and the first; 5.3e-16,
+# 5.0e-16 and 11.1e-16 with cuFFT on the mirrored lines).  The middle bound
+# tells the first from the second, whose single fields vary least.
+@pytest.mark.parametrize("shape,bound", [((16, 513, 16), 1e-15), ((16, 769, 16), 5.2e-16), ((16, 1025, 16), 1.5e-15)])
+def test_cosine_transform_rounding(torch_cuda, shape, bound):
+    from x3div_b200 import Context, to_device, to_host
+    h = np.pi / (shape[1] - 1)
+    lengths = (shape[0] * h, np.pi, shape[2] * h)
+    ctx = Context(*shape, lengths=lengths, bc=(0, 0, 1, 1, 0, 0))
+    errs = []
+    for seed in range(4):
+        g = np.asfortranarray(np.random.default_rng(seed).standard_normal((shape[0], shape[1] - 1, shape[2])))
+        rhs = to_device(g)
+        ctx.poisson(rhs)
+        ctx.sync()
+        want = _walled_y_solution(g, lengths)
+        errs.append(float(np.sqrt(((to_host(rhs) - want)**2).sum() / (want**2).sum())))
+    ctx.close()
+    assert np.mean(errs) < bound, errs

@@ -1,7 +1,8 @@
 """The host side of the pressure solve's tables (poisson_tables.h), checked on
 the CPU through a small C++ program: a context gets every table its lengths
 call for in one block, and none at all where the allocation or the upload
-fails, so that a later solve cannot find some of them missing."""
+fails, so that a later solve cannot find some of them missing; and the roots
+of unity of the cosine transforms are as accurate as doubles can be."""
 import os
 import shutil
 import subprocess
@@ -12,6 +13,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "x3div_b200", "csrc")
 
 HARNESS = r"""
+#include <algorithm>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -55,6 +57,21 @@ int main()
         ok = ok && p.block.size() == end && p.ztw % 2 == 0 && p.xtw % 2 == 0;
         std::printf("layout %d %d %d %d\n", n[0], n[1], n[2], ok ? 1 : 0);
     }
+    // the largest distance of a table entry from its root of unity, in 2^-54
+    auto worst = [](const double *e, int count, long n) {
+        const long double turn = 2 * std::acos(-1.0L);
+        long double w = 0;
+        for (int t = 0; t < count; ++t) {
+            w = std::max(w, std::fabs(e[2 * t] - std::cos(turn * t / n)));
+            w = std::max(w, std::fabs(e[2 * t + 1] + std::sin(turn * t / n)));
+        }
+        return (double)std::ldexp(w, 54);
+    };
+    for (int n = 8; n <= 1024; ++n) {
+        if (!zft_supported(n)) continue;
+        const std::vector<double> y = cosine_tables(n);
+        std::printf("roots %d %.4f\n", n, std::max(worst(&y[0], n, n), worst(&y[2 * n], n, 4L * n)));
+    }
     const std::vector<double> block = {1, 2, 3};
     double *out = nullptr;
     auto place = [&](const char *name, bool full, bool broken, Placed want) {
@@ -85,6 +102,13 @@ def lines(tmp_path_factory):
 def test_every_table_in_its_place(lines):
     got = [ln for ln in lines if ln.startswith("layout")]
     assert len(got) == 6 and all(ln.endswith(" 1") for ln in got), got
+
+
+def test_roots_of_unity_are_rounded_once(lines):
+    """Values below 1 rounded to nearest are within 2^-54; the reference here
+    adds its own long-double rounding, under 2^-60."""
+    got = [float(ln.split()[2]) for ln in lines if ln.startswith("roots")]
+    assert len(got) == 15 and max(got) < 1.02, got
 
 
 def test_a_failure_leaves_no_table(lines):

@@ -245,13 +245,19 @@ __device__ __forceinline__ void zft_stage(double2 *buf, const double2 *tw, const
             const int jm = j % NS;
             // the twiddles W_n^(q jm n / (NS R)), q < R, as powers of w1 (q = 1):
             // one table read a butterfly, each power one product from the last
-            // (a few ulp of W_n after R - 1 products)
+            // (a few ulp of W_n after R - 1 products).  The cosine transforms
+            // along y, which took the place of cuFFT's, read w^1, w^2 and w^4 and
+            // make the others as one product of two: the error of a solve with
+            // walls along y (256 x 129 x 128, 2-norm, six fields) is 6.9e-16 with
+            // these, 7.1e-16 with powers of w^1 and was 6.4e-16 with cuFFT on the
+            // mirrored lines; the solve takes 96 us, 95 with the powers.
             double2 w1 = make_double2(1.0, 0.0);
             if constexpr (NS > 1) {
                 w1 = tw[jm * STRIDE];
                 if (INV) w1.y = -w1.y;
             }
             double2 wq = w1;
+            [[maybe_unused]] double2 wp[R];
 #pragma unroll
             for (int q = 0; q < R; ++q) {
                 const int k = j + q * (N / R);
@@ -267,6 +273,14 @@ __device__ __forceinline__ void zft_stage(double2 *buf, const double2 *tw, const
                 }
                 if (q == 0 || NS == 1) {  // the first stage's twiddles are all 1
                     v[s][q] = x;
+                } else if constexpr (MIR == 3) {
+                    if ((q & (q - 1)) == 0) {
+                        wp[q] = tw[q * jm * STRIDE];
+                        if (INV) wp[q].y = -wp[q].y;
+                    } else {
+                        wp[q] = cmul(wp[q & (q - 1)], wp[q & -q]);
+                    }
+                    v[s][q] = cmul(x, wp[q]);
                 } else {
                     v[s][q] = cmul(x, wq);
                     wq = cmul(wq, w1);
@@ -691,9 +705,9 @@ __global__ void __launch_bounds__(kXftThreads<N>, 1024 / kXftThreads<N>)
         const int l = i % W, k = i / W;  // rows in turn: the shared-memory reads do not conflict
         if (l >= zl.lines) continue;
         const double2 w = __ldg(wt + N + k);
-        const double2 a = cmul(w, zbuf[k * W + l]);
-        const double2 b = cmul(make_double2(w.x, -w.y), zbuf[(k ? N - k : 0) * W + l]);
-        zl.base[(size_t)l * N + k] = make_double2(0.5 * (a.x + b.x), 0.5 * (a.y + b.y));
+        const double2 a = zbuf[k * W + l], b = zbuf[(k ? N - k : 0) * W + l];
+        zl.base[(size_t)l * N + k] = make_double2(0.5 * (w.x * (a.x + b.x) + w.y * (b.y - a.y)),
+                                                  0.5 * (w.x * (a.y + b.y) + w.y * (a.x - b.x)));
     }
 }
 
@@ -1075,18 +1089,7 @@ static int poisson_solve_halves(x3d_ctx_s *mc, double *rhs, const int m[3], cons
         mc->half_spectrum = nullptr;
         return set_error(mc, X3D_ENOMEM, "poisson spectrum");
     }
-    if (half[1] && !mc->d_yft_tw) {
-        const int n = m[1];
-        std::vector<double> tw(4 * (size_t)n);
-        const double pi = std::acos(-1.0);
-        for (int t = 0; t < n; ++t) {
-            tw[2 * t] = std::cos(2.0 * pi * t / n);
-            tw[2 * t + 1] = -std::sin(2.0 * pi * t / n);
-            tw[2 * (n + t)] = std::cos(pi * t / (2.0 * n));
-            tw[2 * (n + t) + 1] = -std::sin(pi * t / (2.0 * n));
-        }
-        if ((rc = place_tables(mc, tw, &mc->d_yft_tw))) return rc;
-    }
+    if (half[1] && !mc->d_yft_tw && (rc = place_tables(mc, cosine_tables(m[1]), &mc->d_yft_tw))) return rc;
     if (!half[1] && !mc->plan_yh_ready) {
         int n = mc->ny;
         if (cufftPlanMany(&mc->plan_yh, 1, &n, nullptr, 1, 0, nullptr, 1, 0, CUFFT_Z2Z, (int)lines) != CUFFT_SUCCESS)

@@ -21,6 +21,36 @@ inline bool zft_supported(int n)
     return false;
 }
 
+// e^{-2 pi i t / n} to within half a unit in the last place: the angle, at most
+// an eighth of a turn, and its sine and cosine in long double.
+inline void unit_root(long t, long n, double *re, double *im)
+{
+    t %= n;
+    const long q = 4 * t / n, r = 4 * t - q * n;  // quarter turns, and r / n of the next
+    const long double half_pi = std::acos(-1.0L) / 2;
+    const bool far = 2 * r > n;
+    const long double a = half_pi * (far ? n - r : r) / n;
+    const double c = (double)(far ? std::sin(a) : std::cos(a)), s = (double)(far ? std::cos(a) : std::sin(a));
+    switch (q) {  // (c, -s) turned q quarters clockwise
+    case 0: *re = c, *im = -s; break;
+    case 1: *re = -s, *im = -c; break;
+    case 2: *re = -c, *im = s; break;
+    default: *re = s, *im = c; break;
+    }
+}
+
+// The tables of the cosine transforms of n points (k_dct_y): e^{-2 pi i t / n},
+// then e^{-i pi k / 2n}, t, k < n.
+inline std::vector<double> cosine_tables(int n)
+{
+    std::vector<double> tw(4 * (size_t)n);
+    for (int t = 0; t < n; ++t) {
+        unit_root(t, n, &tw[2 * t], &tw[2 * t + 1]);
+        unit_root(t, 4L * n, &tw[2 * ((size_t)n + t)], &tw[2 * ((size_t)n + t) + 1]);
+    }
+    return tw;
+}
+
 // (k2, t) of each mode along one direction.
 struct WaveTables {
     std::vector<double> k2, t;
