@@ -321,11 +321,10 @@ void finish_op(OpHost &op)
 // chunks' forward and backward multipliers.  With P_i the product of -s from
 // the chunk's start to i, H_i = w_i P_i - fw_i H_{i+1} and G_i the product of
 // -fw from i to the chunk's end.  Entries past the line's end are zero.
-// Returns the scan depth for thr, or -1 where a factor is not finite or a
+// Returns the scan depth (the fewest chunks any of whose runs multiply to below
+// thr, at most all of them), or -1 where a factor is not finite or a
 // multiplier above 1 would let a carry grow (no operator of the library).
-// uniform: the longest run of whole chunks whose s, w and fw each stay within
-// eps (relative; under the rounding of the type) of their first entry.
-static int build_wall_tables(const OpHost &h, int L, double thr, double eps, std::vector<double> &tab, int uniform[2])
+static int build_wall_tables(const OpHost &h, int L, double thr, std::vector<double> &tab)
 {
     const int n = h.n, C = (n + L - 1) / L, P = C * L;
     tab.assign((size_t)5 * P + 2 * C, 0.0);
@@ -364,8 +363,6 @@ static int build_wall_tables(const OpHost &h, int L, double thr, double eps, std
     return depth;
 }
 
-// Scan depths for chunk length L: smallest k such that any k consecutive
-// chunk multipliers multiply to below 1e-20 (capped at the chunk count).
 int upload_op(x3d_op_s *op)
 {
     const OpHost &h = op->h;
@@ -377,8 +374,8 @@ int upload_op(x3d_op_s *op)
     std::vector<double> wall[2];
     bool walls = !h.periodic;
     if (walls) {
-        op->wall_depth[0] = build_wall_tables(h, kChunkLong<float>, 1e-12, 1e-9, wall[0], op->wall_uniform[0]);
-        op->wall_depth[1] = build_wall_tables(h, kChunkLong<double>, 1e-20, 4e-16, wall[1], op->wall_uniform[1]);
+        op->wall_depth[0] = build_wall_tables(h, kChunkLong<float>, 1e-12, wall[0]);
+        op->wall_depth[1] = build_wall_tables(h, kChunkLong<double>, 1e-20, wall[1]);
         walls = op->wall_depth[0] > 0 && op->wall_depth[1] > 0;
     }
     const size_t o_wf = al(o_d + 5 * n * sizeof(double));

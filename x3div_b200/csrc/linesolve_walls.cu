@@ -28,15 +28,13 @@
 namespace x3d {
 
 // An operator's tables for chunks of L points, P = C L entries a row: s, w,
-// fw, H, G, then the chunks' forward and backward multipliers.  Away from the
-// walls the factors settle: chunks u0 .. u1 - 1 hold one value each of s, w and
-// fw to rounding, read once instead of per point.  depth: chunks
+// fw, H, G, then the chunks' forward and backward multipliers.  depth: chunks
 // a carry scan visits before the product of multipliers is below 1e-20
 // (FP64) or 1e-12 (FP32).
 template <typename T>
 struct WallTables {
     const T *s, *w, *fw, *h, *g, *mf, *mb;
-    int depth, u0, u1;
+    int depth;
 };
 
 // Point k of a line of n_in points, where the staggered stencils reach past
@@ -79,30 +77,21 @@ __device__ __forceinline__ void wall_solve(const WallTables<T> &tb, T (&r)[L], c
         for (int j = 0; j < L; ++j) r[j] = j < nv ? r[j] : T(0);
     }
     T z = T(0), y = T(0);
-    if (c >= tb.u0 && c < tb.u1) {
-        const T se = __ldg(tb.s + cs), we = __ldg(tb.w + cs), fe = __ldg(tb.fw + cs);
 #pragma unroll
-        for (int j = 0; j < L; ++j) r[j] = z = fma(-se, z, r[j]);
-        sc.fz[q] = z;
+    for (int j = 0; j < L; j += V) {
+        const VT sv = __ldg(reinterpret_cast<const VT *>(tb.s + cs + j));
+        const T *se = reinterpret_cast<const T *>(&sv);
 #pragma unroll
-        for (int j = L - 1; j >= 0; --j) r[j] = y = fma(-fe, y, r[j] * we);
-    } else {
+        for (int v = 0; v < V; ++v) r[j + v] = z = fma(-se[v], z, r[j + v]);
+    }
+    sc.fz[q] = z;
 #pragma unroll
-        for (int j = 0; j < L; j += V) {
-            const VT sv = __ldg(reinterpret_cast<const VT *>(tb.s + cs + j));
-            const T *se = reinterpret_cast<const T *>(&sv);
+    for (int j = L - V; j >= 0; j -= V) {
+        const VT wv = __ldg(reinterpret_cast<const VT *>(tb.w + cs + j));
+        const VT fv = __ldg(reinterpret_cast<const VT *>(tb.fw + cs + j));
+        const T *we = reinterpret_cast<const T *>(&wv), *fe = reinterpret_cast<const T *>(&fv);
 #pragma unroll
-            for (int v = 0; v < V; ++v) r[j + v] = z = fma(-se[v], z, r[j + v]);
-        }
-        sc.fz[q] = z;
-#pragma unroll
-        for (int j = L - V; j >= 0; j -= V) {
-            const VT wv = __ldg(reinterpret_cast<const VT *>(tb.w + cs + j));
-            const VT fv = __ldg(reinterpret_cast<const VT *>(tb.fw + cs + j));
-            const T *we = reinterpret_cast<const T *>(&wv), *fe = reinterpret_cast<const T *>(&fv);
-#pragma unroll
-            for (int v = V - 1; v >= 0; --v) r[j + v] = y = fma(-fe[v], y, r[j + v] * we[v]);
-        }
+        for (int v = V - 1; v >= 0; --v) r[j + v] = y = fma(-fe[v], y, r[j + v] * we[v]);
     }
     __syncthreads();
     T F = T(0);
@@ -293,8 +282,6 @@ static int launch_wall_t(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, 
     if constexpr (p == 0) tab = op->wallf, lo = op->opf;
     else tab = op->walld, lo = op->opd;
     tb.depth = op->wall_depth[p];
-    tb.u0 = op->wall_uniform[p][0];
-    tb.u1 = op->wall_uniform[p][1];
     if (!tab) return X3D_EUNSUPPORTED;
     // the chunk stencils take the scalars that the circulant form scales
     lo.ca = lo.a, lo.cb = lo.b, lo.cc = lo.c, lo.cd = lo.d;

@@ -90,7 +90,6 @@ struct x3d_op_s {
     const float *wallf = nullptr;
     const double *walld = nullptr;
     int wall_depth[2] = {0, 0};
-    int wall_uniform[2][2] = {};  // first and last + 1 chunk whose factors are one value each
 };
 
 struct x3d_ctx_s {
