@@ -193,3 +193,38 @@ def test_pressure_one_element_into_its_allocation(oracle, torch_cuda, shape, pre
     with pytest.raises(X3DError):  # a complex array has no such address
         ctx.poisson_zpencil(new(1), 1, 0, 1, 0)
     ctx.close()
+
+
+# x_tile_lines: 8 lines a tile, 16, and (FP32) 32
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("shape", [(17, 12, 10), (17, 160, 130), (17, 300, 260), (33, 20, 30), (9, 130, 150)])
+def test_short_x_lines(oracle, torch_cuda, shape, prec):
+    """Periodic and walled x operators on lines of one or two chunks."""
+    torch = torch_cuda
+    from x3div_b200 import Context, to_device, to_host
+    dt_ = torch.float64 if prec == "f64" else torch.float32
+    tol = 1e-12 if prec == "f64" else 1e-5
+    u = to_device(seeded_field(shape, 3, lengths=LEN, noise=1e-2), dt_)
+    used = to_host(u).astype(np.float64)
+    ctx = Context(*shape, lengths=LEN, precision=prec)
+    names = [("derx", "der"), ("derxx", "der2"), ("derxvp", "dervp"), ("derxpv", "derpv"), ("intxvp", "intvp"),
+             ("intxpv", "intpv")]
+    outs = [torch.full_like(u, float("nan")) for _ in names]
+    one = torch.full_like(u, float("nan"))
+    ctx.apply_batch([(ctx.op(n), u, o) for (n, _), o in zip(names, outs)])
+    ctx.derx(one, u, ctx.op("derx"), *shape)
+    ctx.sync()
+    for (_, kind), o in zip(names, outs):
+        assert rel_err(to_host(o), oracle.apply(kind, X, used, ctx.dx)) < tol, kind
+    assert rel_err(to_host(one), oracle.apply("der", X, used, ctx.dx)) < tol
+    ctx.close()
+    n = shape[0]
+    ctx = Context(*shape, lengths=LEN, precision=prec, bc=(2, 1, 0, 0, 0, 0))
+    t = torch.full_like(u, float("nan"))
+    ctx.derx(t, u, ctx.op("derx"), *shape)
+    s = torch.full((shape[2], shape[1], n - 1), float("nan"), dtype=dt_, device="cuda")
+    ctx.interxvp(s, u, ctx.op("intxvp"), n, n - 1, *shape[1:])
+    ctx.sync()
+    assert rel_err(to_host(t), oracle.der_np(X, used, ctx.dx, 2, 1, 0)) < tol
+    assert rel_err(to_host(s), oracle.stag_np("intvp", X, used, ctx.dx, 2, 1, 1)) < tol
+    ctx.close()

@@ -713,8 +713,13 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                     // short last chunk does not run beside a full one in the
                     // same warp (250 x 171 x 129 sweep 189 -> 155 us; FP64
                     // lines of that length do not fit)
+                    const bool wide = W == 16 && sizeof(T) == 4 && !acc && C * 32 <= 256;
+                    int lines = wide ? 32 : W;
+                    if (W == 16 && dir == DX) lines = x_tile_lines(lines, C, (long)ny * nz, ctx->num_sms, es);
+                    if constexpr (W == 16)
+                        if (lines == 8) return launch_stage_any<T, 8>(ctx, prog, acc, dir, nx, ny, nz);
                     if constexpr (W == 16 && sizeof(T) == 4)
-                        if (!acc && C * 32 <= 256) {
+                        if (lines == 32) {
                             const int rc = launch_stage_any<T, 32>(ctx, prog, acc, dir, nx, ny, nz);
                             if (rc != X3D_EUNSUPPORTED) return rc;
                         }

@@ -114,6 +114,26 @@ inline bool program_acc(const StageProgram<T> &p)
     return false;
 }
 
+// Lines per CTA for x lines of C chunks whose rows every warp copies in turn
+// (linesolve_any.cu, linesolve_walls.cu), at most `widest`.  A tile of one or
+// two chunks is one or two warps, which take 32 or 16 rows each: where few such
+// warps share an SM that is the launch's time, and 8 lines a CTA (8 rows a warp,
+// most of its lanes idle in the solve) are faster, up to the number of warps at
+// which the idle lanes cost as much.  FP32, 17 points, one operator: 600 lines
+// 10.8 us on 32 lines, 5.0 on 8; 16384 lines 11.5 and 9.2; 40000 lines (8 warps
+// an SM) walls 15.3 on 32, 10.9 on 16, 13.4 on 8; 90000 lines 16.5 on 32, 18.7
+// on 16.  Two chunks: FP64 17 points, 16384 lines (7 warps an SM) 9.1 and 7.6,
+// 40000 lines 10.0 and 12.8; FP32 33 points, 4096 lines 7.1 and 5.6, 8000 lines
+// (3.4 warps) 7.5 and 7.8.
+inline int x_tile_lines(int widest, int C, long lines, int num_sms, size_t es)
+{
+    const int warps = (C * widest + 31) / 32, rows = widest / warps;
+    const double per_sm = (double)((lines + widest - 1) / widest * warps) / num_sms;
+    if (rows >= 32) return per_sm < 4.0 ? 8 : (per_sm < 16.0 ? 16 : widest);
+    if (rows >= 16 && per_sm < (es == 8 ? 8.0 : 2.5)) return 8;
+    return widest;
+}
+
 // The same program on a grid whose rows or addresses are not whole 16-byte
 // units, W lines per CTA in chunks of kChunkLong<T> points (linesolve_any.cu);
 // launch_stage's configurations 0 (W = 16) and 3 (W = 8) fall through to it.

@@ -322,8 +322,9 @@ static int launch_wall_t(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, 
                                           o1, o2, dir, refl, C, vec),
                           "ls_wall_yz launch");
     };
-    int rc = run(std::integral_constant<int, 32>{});
-    if (rc == X3D_EUNSUPPORTED) rc = run(std::integral_constant<int, 16>{});
+    const int lines = dir == DX ? x_tile_lines(32, C, (long)o1 * o2, ctx->num_sms, sizeof(T)) : 32;
+    int rc = lines == 32 ? run(std::integral_constant<int, 32>{}) : X3D_EUNSUPPORTED;
+    if (rc == X3D_EUNSUPPORTED && lines >= 16) rc = run(std::integral_constant<int, 16>{});
     if (rc == X3D_EUNSUPPORTED) rc = run(std::integral_constant<int, 8>{});
     return rc;
 }
