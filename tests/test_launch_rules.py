@@ -58,3 +58,37 @@ def test_x_tiles_are_narrow_only_for_short_lines(run):
     assert [got[32, 4, 1, n] for n in (600, 16384, 40000, 90000)] == [8, 8, 16, 32]
     assert [got[32, 4, 2, n] for n in (600, 4096, 8000)] == [8, 8, 32]
     assert [got[16, 8, 2, n] for n in (600, 16384, 20800)] == [8, 8, 16]
+
+
+PICKS = r"""
+#include <cstdio>
+#include "linesolve_chunk.h"
+using namespace x3d;
+int main()
+{
+    // a rule that names its arguments, asked for many more keys than slots, in
+    // runs and interleaved, each twice
+    CfgPicks<64> picks;
+    long asked = 0, weighed = 0, wrong = 0;
+    auto ask = [&](int dir, int nx, int ny, int nz, int nops, int acc) {
+        const CfgKey k{{8, dir, nx, ny, nz, 1, nops, acc, 0, 148}};
+        const int want = ((dir * 7 + nx) * 1009 + ny * 13 + nz) * 12 + nops * 2 + acc;
+        for (int r = 0; r < 2; ++r) {
+            const DefaultCfgs d = picks.get(k, [&] { ++weighed; return DefaultCfgs{1, {want}}; });
+            ++asked;
+            wrong += d.count != 1 || d.cfg[0] != want;
+        }
+    };
+    for (int pass = 0; pass < 3; ++pass)
+        for (int nx = 8; nx < 40; ++nx)
+            for (int dir = 0; dir < 3; ++dir)
+                for (int nops = 1; nops <= 6; ++nops) ask(dir, nx, 48 - nx, 10 + pass, nops, nops & 1);
+    std::printf("%ld %ld %ld\n", asked, weighed, wrong);
+    return 0;
+}
+"""
+
+
+def test_kept_picks_are_the_rule(run):
+    asked, weighed, wrong = map(int, run("picks", PICKS)[0].split())
+    assert wrong == 0 and weighed == asked // 2  # new keys throughout: the second of each pair is kept

@@ -962,8 +962,8 @@ static double stage_cost(const StageShape &s, size_t es, int dir, int ntiles, in
     return 2.0 + full * wave(s.per_sm) + (rest ? wave((rest + num_sms - 1) / num_sms) : 0.0);
 }
 
-DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
-                         int num_sms)
+static DefaultCfgs weigh_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
+                              int num_sms)
 {
     const bool f32 = es == 4;
     if ((size_t)nx * ny * nz * es > (size_t)24 << 20) {
@@ -991,6 +991,14 @@ DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles,
     if (base < 0) return {1, {0}};
     if (tbest < 0.9 * tbase) return {2, {best, base}};
     return {1, {base}};
+}
+
+DefaultCfgs default_cfgs(size_t es, int dir, int nx, int ny, int nz, int ntiles, int nops, bool acc, bool in64,
+                         int num_sms)
+{
+    thread_local CfgPicks<64> picks;
+    return picks.get({{(int)es, dir, nx, ny, nz, ntiles, nops, acc, in64, num_sms}},
+                     [&] { return weigh_cfgs(es, dir, nx, ny, nz, ntiles, nops, acc, in64, num_sms); });
 }
 
 template <typename T>
