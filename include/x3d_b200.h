@@ -267,7 +267,7 @@ int x3d_apply(x3d_ctx ctx, x3d_op op, const void *in, void *out);
  * stage of the Euler step (transeq + int_time, divergence, gradp + cor_vel,
  * per direction).  Synchronous; uses context scratch fields (up to 14 of
  * nx*ny*nz doubles); not callable during stream capture.  Without it a
- * fixed default configuration is used.  No reference counterpart. */
+ * rule picks one by the launch's size and program.  No reference counterpart. */
 int x3d_autotune(x3d_ctx ctx, int max_group);
 /* Force kernel configuration cfg (0..5 chunked, one CTA per tile;
  * 6..11 the same shapes as persistent double-buffered kernels; 12..15 y/z
@@ -400,14 +400,20 @@ int x3d_copy_blocks(x3d_ctx ctx, void *dst, const void *src, int elem_bytes, con
  * cosine modes of waves()'s bc = 1 tables (:539-553, :573-588, :603-613),
  * which x3div itself stops on (:104-108).  It is solved as the periodic
  * problem on the box mirrored about both walls of every such direction
- * (2 nxm points over 2 xlx) and cut back: the mirrored field holds exactly
- * those cosine modes.  The first call makes the mirrored box's periodic
- * context and right-hand side (kept until x3d_ctx_destroy).  Where nz and
- * nx / 2 are both 2^p 3^q from 8 to 1024 (nx even), the periodic solve is
- * five launches: the library's x transforms (real lines to a spectrum with
- * y fastest), batched 1-D cuFFT transforms along y, the fused z transform
- * and mode division, and back; the stage choice "poisson_x" = 0
- * (x3d_ctx_set_stage_choice) takes cuFFT's 2-D (x, y) transforms instead. */
+ * (2 nxm points over 2 xlx), whose field holds exactly those cosine modes.
+ * The first call makes the mirrored box's periodic context (kept until
+ * x3d_ctx_destroy).  Where nz and nx / 2 are both 2^p 3^q from 8 to 1024 (nx
+ * even), the periodic solve is five launches: the library's x transforms
+ * (real lines to a spectrum with y fastest), batched 1-D cuFFT transforms
+ * along y, the fused z transform and mode division, and back; the stage
+ * choice "poisson_x" = 0 (x3d_ctx_set_stage_choice) takes cuFFT's 2-D (x, y)
+ * transforms instead.  Between walls the same holds for the mirrored lengths
+ * (nxm for nx / 2, 2 nzm for nz), and with walls in y for nym, along which the
+ * library's cosine transforms take cuFFT's place: the first half of each
+ * mirrored line is all that is stored.  Other lengths, and a rhs off a
+ * 16-byte boundary, are mirrored into a field of the context's (made on the
+ * first such call) and cut back.  A periodic rhs at such an address is copied
+ * to an aligned field of the context's and back. */
 int x3d_poisson(x3d_ctx ctx, double *rhs);
 /* The z part of poisson_000 for a box whose y rows are spread over ranks:
  * spec is this rank's block of the x-y transformed half spectrum (complex

@@ -8,8 +8,8 @@ from conftest import rel_err, seeded_field
 
 pytestmark = pytest.mark.gpu
 
-# (18, 12, 10): x not a multiple of 4, so the fused stage kernels step aside
-# for the one-launch-per-operator composition.
+# (18, 12, 10): in FP32 its rows are 72 bytes, so the fused stages run on tiles
+# copied element by element.
 SHAPES = [(16, 16, 16), (24, 20, 12), (32, 32, 32), (18, 12, 10)]
 LEN = (2 * np.pi, 1.5, 3.0)
 

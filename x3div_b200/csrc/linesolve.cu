@@ -25,9 +25,10 @@
 //               thread reading its own row with 16-byte vectors is bank
 //               conflict free; results are written back in place and stored
 //               with 1-D bulk copies.
-//   ls_generic: any shape/alignment (odd sizes, unaligned pointers, lines
-//               too long for shared memory); one thread per line straight
-//               from global memory.  Correctness path, not a fast path.
+//   ls_generic: any shape/alignment; one thread per line straight from global
+//               memory.  What the chunked kernels do not take (configuration 16
+//               on odd rows, unaligned or in-place fields, lines too long for
+//               shared memory).  Correctness path, not a fast path.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 

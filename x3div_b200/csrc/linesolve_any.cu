@@ -6,7 +6,7 @@
 //
 // What bounds these launches is still HBM: an element copy costs one
 // instruction per 32 elements and input, against some twenty per point and
-// operator for the solve.  Before, such grids went one thread per line through
+// operator for the solve (short x lines excepted, see x_tile_lines).  Before, such grids went one thread per line through
 // global memory (ls_generic), where a warp's 32 x lines touch 32 rows at
 // once; the figures are at launch_stage_any.
 //
@@ -247,9 +247,13 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
 }
 
 // The derivative sweep (18 operators of one field, three launches) took 1547 us
-// at 171 x 129 x 150 FP64 on ls_generic and takes 182 us here (2.8 TB/s of one
-// read per direction and the outputs; 170 with the shifted twins); 1575 and 155
-// us at 250 x 171 x 129 FP32.
+// at 171 x 129 x 150 FP64 on ls_generic and takes 170 us here (3.3 TB/s of one
+// read per direction and the outputs); 1575 and 157 us at 250 x 171 x 129 FP32.
+// The periodic correction, an FP64 sum there, is the carry scan in the program's
+// type here; the errors against 64 bits are no larger (FP32, 2-norm, rms over 21
+// lines of 17 to 255 points a kind: der 1.13e-7 there, 0.97e-7 here, der2 6.9e-8
+// and 6.8e-8, dervp 7.0e-8 and 5.9e-8, interpvp 9.9e-7 and 8.7e-7; FP64 der
+// 1.30e-15 both, dervp 1.42e-15 and 1.44e-15, interpvp 2.2e-15 and 1.9e-15).
 // prog: its responses filled for chunks of kChunkLong<T> points (launch_stage
 // did), acc: it needs the accumulator or a general flush.
 template <typename T, int W>

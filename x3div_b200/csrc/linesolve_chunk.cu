@@ -711,8 +711,11 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                     // FP32: 32 lines a tile where plain programs still fit 256
                     // threads.  A warp then holds one chunk of 32 lines, so a
                     // short last chunk does not run beside a full one in the
-                    // same warp (250 x 171 x 129 sweep 189 -> 155 us; FP64
-                    // lines of that length do not fit)
+                    // same warp (250 x 171 x 129 sweep 189 -> 155 us; six y
+                    // operators 10.9 us against 15.4 with 16 lines at 65^3, 18.9
+                    // and 26.0 at 97^3, 173 and 229 at 255^3; behind only where
+                    // a last tile of a column or so adds a fourth, 29.0 and 24.3
+                    // at 129^3; FP64 lines of that length do not fit)
                     const bool wide = W == 16 && sizeof(T) == 4 && !acc && C * 32 <= 256;
                     int lines = wide ? 32 : W;
                     if (W == 16 && dir == DX) lines = x_tile_lines(lines, C, (long)ny * nz, ctx->num_sms, es);
@@ -893,18 +896,24 @@ static int launch_stage_sel(x3d_ctx_s *ctx, const StageProgram<T> &prog, int dir
 //
 // Fields above 24 MiB fill the SMs many times over, and the order is the same
 // for all of them: the kernels built for three CTAs per SM for plain programs
-// (384^3 FP64, six y operators: 673 us on 19, 1051 on 0; 256^3 FP32 y 113 on
-// 20, 127 on 0), pairs of lines a thread for FP32 y/z momentum (256^3 z 198 on
+// (384^3 FP64, six y operators: 541 us on 19, 889 on 0; 256^3 FP32 y 92 on
+// 20, 106 on 0), pairs of lines a thread for FP32 y/z momentum (256^3 z 198 on
 // 14, 236 on 0), 8-line tiles for FP64 x programs that accumulate, whose three
 // staged fields then fit more CTAs (256^3 momentum x 313 on 3, 460 on 0).
 //
 // Below that what matters is how the tiles of a configuration divide into
 // waves, and no line through the sizes holds: stage_cost estimates each
 // configuration's time from its waves, and one that comes out at least a tenth
-// below the long-chunk default replaces it.  Over the measured launches the
-// pick is on average 4 % behind the fastest configuration and 19 % ahead of the
-// default (64^3 FP32, six y operators: 8.6 us on 4 against 17.9 on 0; 16 x 176
-// x 128 FP64 z, where the short chunk would take a second wave, stays on 0).
+// below the long-chunk default replaces it.  It was fitted before derpv and
+// interpv became second outputs of their twins' solves; over 270 launches since
+// (22 boxes up to 24 MiB, one and six operators) the pick is on average 4 and 5 %
+// behind the fastest configuration and 9 and 18 % ahead of 0 (64^3 FP32, six y
+// operators: 7.6 us on 2, 7.3 on 4, 10.7 on 0), at worst 40 % behind (112^3
+// FP32 along y: 19.9 us on the picked, 14.2 on 0).  nops counts every operator
+// of the list, whether or not it gets a solve of its own; counting solves
+// instead picks the same.  Rows that are not whole 16-byte units are the business
+// of linesolve_any.cu, reached through configuration 0 or 3, whichever of the
+// pick or the order after it comes first.
 //
 // The persistent configurations are left to the autotuner, although 17 is up
 // to 8 % ahead of 20: they claim tiles from the context's one counter, and an

@@ -1041,7 +1041,7 @@ int poisson_zpencil(x3d_ctx_s *ctx, void *spec, int nxl, int i0, int ny_loc, int
 // with walls in y, its m points), nothing is mirrored in memory: the x and z
 // transforms read and write the first half of each mirrored line and y takes a
 // cosine transform (poisson_solve_halves; 256 x 129 x 128 with walls in y: 204 us
-// before, 106 now).  Otherwise the box is mirrored and cut back, one pass each, around the
+// before, 96 now).  Otherwise the box is mirrored and cut back, one pass each, around the
 // library's periodic solve.
 
 // ext (Mx, My, Mz) from p (mx, my, mz): M = 2m along a mirrored direction,
