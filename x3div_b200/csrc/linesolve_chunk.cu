@@ -86,7 +86,13 @@ struct StageMaps {
 // FP32 16-line, 32-point-chunk kernel fits 80 registers without spilling, so
 // an SM holds 24 warps instead of 16 -- the sweep kernels are latency- and
 // issue-bound at 16 (issue active about half the cycles).
-template <typename T, int W, int L, bool ACC, bool PERSIST, int PR = 1, int OCC = 1, typename TI = T>
+//
+// SHIFT: the plain kernel for programs with shifted second outputs (StageOp::
+// shift_out).  Programs without run the kernel without that code: compiled in and
+// unused it cost 512^3 launches of one operator 4 to 8 % (FP32 y, configuration
+// 17, 167 -> 180 us; FP64 x, configuration 9, 381 -> 400).
+template <typename T, int W, int L, bool ACC, bool PERSIST, int PR = 1, int OCC = 1, typename TI = T,
+          bool SHIFT = false>
 __global__ void __launch_bounds__(OCC > 1 ? 256 : kStageThreads<T, L, PR>, OCC)
     ls_stage_yz(const __grid_constant__ StageMaps maps, const __grid_constant__ StageProgram<T> prog, int nx,
                 int ny, int dir, int box_n, int nbox, int tma_halo, size_t tile_bytes, long ntiles,
@@ -228,8 +234,9 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : kStageThreads<T, L, PR>, OCC)
                 if (so.flush && live) flush_yz<T, V, L, true>(flush_args(so), acc, obase, ostride, nv);
             } else {
                 if (so.flush && live) flush_yz<T, V, L, false>(flush_args(so), r, obase, ostride, nv);
-                if (so.shift_out && live)
-                    flush_yz_shifted<T, V, L>(so.shift_out, r, obase, cs, ostride, nv, c == C - 1);
+                if constexpr (SHIFT)
+                    if (so.shift_out && live)
+                        flush_yz_shifted<T, V, L>(so.shift_out, r, obase, cs, ostride, nv, c == C - 1);
             }
         }
         if (!PERSIST) break;
@@ -472,7 +479,8 @@ __device__ __forceinline__ void fill_halos_x(unsigned char *base, size_t tile_by
     }
 }
 
-template <typename T, int W, int L, bool ACC, bool PERSIST, int OCC = 1>
+// SHIFT as for ls_stage_yz.
+template <typename T, int W, int L, bool ACC, bool PERSIST, int OCC = 1, bool SHIFT = false>
 __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
     ls_stage_x(const __grid_constant__ StageProgram<T> prog, long nlines, int pitch, size_t tile_bytes,
                long ntiles, unsigned long long *claim, int *err)
@@ -604,7 +612,8 @@ __global__ void __launch_bounds__(OCC > 1 ? 256 : 512, OCC)
                 if (so.flush) flush_x_staged<T, L, false>(flush_args(so), r, out_s, l, l0, rows, pitch, n, cs, nv);
                 // from the staging rows, which the next operator writes only
                 // after its solve's barriers
-                if (so.shift_out) flush_rows_shifted<T, true>(so.shift_out, out_s, l0, rows, pitch, n);
+                if constexpr (SHIFT)
+                    if (so.shift_out) flush_rows_shifted<T, true>(so.shift_out, out_s, l0, rows, pitch, n);
             }
         }
         if (!PERSIST) break;
@@ -692,6 +701,8 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         // the ACC kernels carry the accumulator and every flush form; the
         // others only plain operators (out = the solve)
         const bool acc = program_acc(prog);
+        bool shift = false;  // plain programs only (plain_program)
+        for (int k = 0; k < prog.nops; ++k) shift = shift || prog.ops[k].shift_out;
         const int n = prog.ops[0].op.n;
         for (int k = 0; k < prog.nops; ++k)
             if (!prog.ops[k].op.circ || prog.ops[k].op.n != n) return X3D_EUNSUPPORTED;
@@ -756,7 +767,7 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
                                 (size_t)W * pitch * es;
             if (smem + 1024 > ctx->smem_optin) return X3D_EUNSUPPORTED;
             fill_resp(prog, L, n);
-            auto kern = ls_stage_x<T, W, L, false, PERSIST, OCC>;
+            auto kern = shift ? ls_stage_x<T, W, L, false, PERSIST, OCC, true> : ls_stage_x<T, W, L, false, PERSIST, OCC>;
             if constexpr (OCC == 1)  // the OCC > 1 kernels take plain programs only
                 if (acc) kern = ls_stage_x<T, W, L, true, PERSIST>;
             cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -816,7 +827,8 @@ static int launch_stage_cfg(x3d_ctx_s *ctx, const StageProgram<T> &prog_in, int 
         prog.prefetch_mask = 0;
         for (int k = 0; k < prog.nops; ++k)
             if (prog.ops[k].prefetch_base) prog.prefetch_mask |= 1 << k;
-        auto kern = ls_stage_yz<T, W, L, false, PERSIST, PR, OCC>;
+        auto kern = shift ? ls_stage_yz<T, W, L, false, PERSIST, PR, OCC, T, true>
+                          : ls_stage_yz<T, W, L, false, PERSIST, PR, OCC>;
         if constexpr (OCC == 1)  // the OCC > 1 kernels take plain programs only
             if (acc) kern = ls_stage_yz<T, W, L, true, PERSIST, PR, OCC>;
         if constexpr (std::is_same<T, float>::value && PR == 1 && OCC == 1)
