@@ -125,3 +125,34 @@ def test_batch_jobs_of_one_shape_with_different_twins(oracle, torch_cuda, prec, 
                     ref = oracle.apply(kind, d, used, 2 * np.pi / b[d])
                     assert rel_err(to_host(os_[f][d][k]), ref) < tol, (b, f, d, kind)
     batch.close()
+
+
+@pytest.mark.parametrize("prec", ["f64", "f32"])
+@pytest.mark.parametrize("tuned", [False, True])
+@pytest.mark.parametrize("nops", [1, 3, 4, 5])
+def test_batch_of_fewer_families(oracle, torch_cuda, prec, nops, tuned):
+    """Lists without a twin run the batch kernel without the shifted outputs
+    (1 and 3 families), lists with one the kernel with them."""
+    torch = torch_cuda
+    from x3div_b200 import Batch, to_device, to_host
+    boxes = [(64, 48, 32), (100, 36, 20), (40, 8, 140)]
+    dt = torch.float64 if prec == "f64" else torch.float32
+    fields = [[to_device(seeded_field(b, seed=i, noise=1e-2), dt)] for i, b in enumerate(boxes)]
+    outs = [[[[torch.full_like(fs[0], float("nan")) for _ in range(6)] for _ in range(3)]] for fs in fields]
+    batch = Batch(boxes, precision=prec)
+    batch.bind_sweep(fields, outs, nops)
+    if tuned:
+        batch.autotune()
+    batch.run()
+    batch.sync()
+    tol = 1e-12 if prec == "f64" else 1e-5
+    for b, fs, os_ in zip(boxes, fields, outs):
+        used = to_host(fs[0]).astype(np.float64)
+        for d in range(3):
+            for k, kind in enumerate(("der", "der2", "dervp", "derpv", "intvp", "intpv")):
+                got = to_host(os_[0][d][k])
+                if k < nops:
+                    assert rel_err(got, oracle.apply(kind, d, used, 2 * np.pi / b[d])) < tol, (b, d, kind)
+                else:
+                    assert np.isnan(got).all()
+    batch.close()

@@ -1095,7 +1095,7 @@ __host__ __device__ constexpr size_t batch_out_offset(size_t tile_cap)
 // x outputs either go straight out as each thread's 16-byte vectors or, for
 // jobs with xstage set, are staged in shared-memory rows (out_s, the tile's
 // pitch) and leave as one bulk copy per row, as in ls_stage_x.
-template <typename T, int L, bool XS>
+template <typename T, int L, bool XS, bool SHIFT>
 __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, T *out_s, const T *resp_s,
                                            const ChunkScratch<T> &scf, int t, long l0, int rows, int x0, int o)
 {
@@ -1144,7 +1144,7 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                         }
                     }
                 }
-                if (J.shift_out[k]) {
+                if (SHIFT && J.shift_out[k]) {
                     // one point on: the chunk's first point is the end of the
                     // chunk before, passed through the scratch that held the
                     // forward ends (read before the solve's second barrier)
@@ -1192,7 +1192,8 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                            (uint32_t)(n * sizeof(T)));
                 bulk_commit();
             }
-            if (J.shift_out[k]) flush_rows_shifted<T, true>(J.shift_out[k], out_s, l0, rows, J.pitch, n);
+            if (SHIFT && J.shift_out[k])
+                flush_rows_shifted<T, true>(J.shift_out[k], out_s, l0, rows, J.pitch, n);
         }
     } else {
         const T *col = tile + (size_t)(J.halo + cs - 4) * W + l;  // points cs-4 .. cs+L+3
@@ -1225,7 +1226,7 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
                         dst += ostride;
                     }
                 }
-                if (J.shift_out[k])
+                if (SHIFT && J.shift_out[k])
                     flush_yz_shifted<T, T, L>(J.shift_out[k], r, obase, cs, ostride, nv, c == C - 1);
             }
         }
@@ -1240,7 +1241,7 @@ __device__ __forceinline__ void batch_item(const BatchJob<T> &J, const T *tile, 
 template <typename T>
 constexpr int kBatchHdrVecs = (int)((offsetof(BatchJob<T>, resp) + 15) / 16);
 
-template <typename T, int VAR>
+template <typename T, int VAR, bool SHIFT>
 __global__ void __launch_bounds__(kBatchThreads, 2)
     ls_batch(const BatchJob<T> *__restrict__ jobs, int njobs, long total,
              unsigned long long *counter, size_t tile_cap, int *err)
@@ -1374,9 +1375,9 @@ __global__ void __launch_bounds__(kBatchThreads, 2)
         if (s_item < total) copy_header(s_job, slot ^ 1);
         constexpr bool XS = VAR == kBatchStaged;
         if (VAR == kBatchLong || J.L == kChunkLong<T>)
-            batch_item<T, kChunkLong<T>, XS>(J, tile, out_s, resp_s, scf, t, l0, rows, x0, o);
+            batch_item<T, kChunkLong<T>, XS, SHIFT>(J, tile, out_s, resp_s, scf, t, l0, rows, x0, o);
         else
-            batch_item<T, kChunkShort<T>, XS>(J, tile, out_s, resp_s, scf, t, l0, rows, x0, o);
+            batch_item<T, kChunkShort<T>, XS, SHIFT>(J, tile, out_s, resp_s, scf, t, l0, rows, x0, o);
     }
     if (VAR == kBatchStaged) bulk_wait_all();  // x rows in flight (issued by this thread)
 }
@@ -1453,27 +1454,32 @@ bool plan_batch_job(BatchJob<T> &J, int L, int w_req, int xstage, size_t *tile_b
 template <typename T>
 size_t batch_smem_bytes(size_t tile_cap, int variant)
 {
-    return variant == kBatchStaged ? batch_out_offset<T>(tile_cap) + tile_cap
-                                   : 2 * tile_cap + batch_scratch_bytes_c<T>();
+    return (variant & 3) == kBatchStaged ? batch_out_offset<T>(tile_cap) + tile_cap
+                                         : 2 * tile_cap + batch_scratch_bytes_c<T>();
 }
 
 template <typename T>
 static void (*batch_kernel(int variant))(const BatchJob<T> *, int, long, unsigned long long *, size_t, int *)
 {
-    if (variant == kBatchStaged) return ls_batch<T, kBatchStaged>;
-    if (variant == kBatchMixed) return ls_batch<T, kBatchMixed>;
-    return ls_batch<T, kBatchLong>;
+    const bool shift = variant & kBatchShift;
+    switch (variant & 3) {
+    case kBatchStaged: return shift ? ls_batch<T, kBatchStaged, true> : ls_batch<T, kBatchStaged, false>;
+    case kBatchMixed: return shift ? ls_batch<T, kBatchMixed, true> : ls_batch<T, kBatchMixed, false>;
+    default: return shift ? ls_batch<T, kBatchLong, true> : ls_batch<T, kBatchLong, false>;
+    }
 }
 
 template <typename T>
 int batch_variant(const BatchJob<T> *jobs, int njobs)
 {
-    int v = kBatchLong;
+    int v = kBatchLong, shift = 0;
     for (int i = 0; i < njobs; ++i) {
-        if (jobs[i].dir == DX && jobs[i].xstage) return kBatchStaged;
-        if (jobs[i].L != kChunkLong<T>) v = kBatchMixed;
+        if (jobs[i].dir == DX && jobs[i].xstage) v = kBatchStaged;
+        else if (jobs[i].L != kChunkLong<T>) v = std::max(v, (int)kBatchMixed);
+        for (int k = 0; k < jobs[i].nops; ++k)
+            if (jobs[i].shift_out[k]) shift = kBatchShift;
     }
-    return v;
+    return v | shift;
 }
 
 template <typename T>

@@ -210,9 +210,11 @@ bool plan_batch_job(BatchJob<T> &J, int L, int w_req, int xstage, size_t *tile_b
 
 // Variants of the batch kernel: every job on the long chunk with x outputs
 // straight out; each job's own chunk length; and x outputs staged in shared
-// memory where a job sets xstage.  batch_variant picks the narrowest one a
-// host job list needs.
-enum BatchVariant { kBatchLong = 0, kBatchMixed = 1, kBatchStaged = 2 };
+// memory where a job sets xstage; each with and without (kBatchShift) shifted
+// second outputs, whose code costs lists that never run it 2 % (five boxes, FP32,
+// three operators: 390 us, 380 without).  batch_variant picks the narrowest one
+// a host job list needs.
+enum BatchVariant { kBatchLong = 0, kBatchMixed = 1, kBatchStaged = 2, kBatchShift = 4 };
 template <typename T>
 int batch_variant(const BatchJob<T> *jobs, int njobs);
 
