@@ -1,6 +1,6 @@
 // Batches of independent periodic boxes of uneven sizes: the derivative
 // sweep of every box in one persistent launch (BatchJob work-list, see
-// linesolve_chunk.cu), capturable as a CUDA graph.  Boxes of one shape share
+// linesolve_batch.cu), capturable as a CUDA graph.  Boxes of one shape share
 // a context, hence its FP64 operator precompute.
 #include <cuda_runtime.h>
 

@@ -1,5 +1,5 @@
 // Device code of the chunked line solves shared by the stage kernels
-// (linesolve_chunk.cu: TMA and bulk-copied tiles; linesolve_any.cu: tiles of
+// (linesolve_chunk.cu and linesolve_batch.cu: TMA and bulk-copied tiles; linesolve_any.cu: tiles of
 // any extent and alignment): stencils on a chunk's window, the chunk solve
 // with its two carry exchanges, the accumulator and the flushes of y/z
 // chunks.  The solve itself is described at the top of linesolve_chunk.cu.
@@ -139,6 +139,8 @@ __device__ __forceinline__ void chunk_rhs(int kind, const Load &load, T (&r)[L],
 // the last chunk's window exist but hold values that are never used.
 constexpr int kHalo = 4;
 
+constexpr uint64_t kChunkWaitNs = 2000000000ull;  // bounded waits on a tile's copies: 2 s
+
 // Fills the halos of ntiles staged y/z tiles of W columns whose point i sits
 // in row h0 + i: rows h0-4 .. h0-1 from points n-4 .. n-1, rows h0+n ..
 // h0+n+3 from points 0 .. 3.
@@ -154,6 +156,46 @@ __device__ __forceinline__ void fill_halos_yz(unsigned char *base, size_t tile_b
         const int dst = h < 4 ? h0 - 4 + h : h0 + n + h - 4;
         const int src = h < 4 ? h0 + n - 4 + h : h0 + h - 4;
         tp[dst * W + x] = tp[src * W + x];
+    }
+}
+
+// 16-byte vector of T.
+template <typename T>
+struct Vec4;
+template <>
+struct Vec4<float> {
+    static constexpr int N = 4;
+    using type = float4;
+};
+template <>
+struct Vec4<double> {
+    static constexpr int N = 2;
+    using type = double2;
+};
+template <>
+struct Vec4<F2> {
+    static constexpr int N = 2;
+    using type = float4;
+};
+
+// Fills the halos of ntiles staged x tiles of `rows` padded rows whose
+// point i sits at element kHalo + i: elements 0 .. 3 from points n-4 .. n-1,
+// elements n+4 .. n+7 from points 0 .. 3, moved as 16-byte vectors.
+template <typename T>
+__device__ __forceinline__ void fill_halos_x(unsigned char *base, size_t tile_bytes, int ntiles, int rows,
+                                             int pitch, int n)
+{
+    using VT = typename Vec4<T>::type;
+    constexpr int V = Vec4<T>::N;
+    constexpr int per_row = 8 / V;
+    const int per = rows * per_row;
+    for (int i = threadIdx.x; i < per * ntiles; i += blockDim.x) {
+        const int ti = i / per, r = i - ti * per;
+        const int rr = r / per_row, h = (r - rr * per_row) * V;
+        T *row = reinterpret_cast<T *>(base + ti * tile_bytes) + (size_t)rr * pitch;
+        const int dst = h < 4 ? h : n + h;
+        const int src = h < 4 ? n + h : h;
+        *reinterpret_cast<VT *>(row + dst) = *reinterpret_cast<const VT *>(row + src);
     }
 }
 
@@ -205,25 +247,6 @@ __device__ __forceinline__ T chunk_carry(const T *e, int K, T mf, T ml, T wrap, 
     }
     return full ? carry * wrap : carry;
 }
-
-// 16-byte vector of T.
-template <typename T>
-struct Vec4;
-template <>
-struct Vec4<float> {
-    static constexpr int N = 4;
-    using type = float4;
-};
-template <>
-struct Vec4<double> {
-    static constexpr int N = 2;
-    using type = double2;
-};
-template <>
-struct Vec4<F2> {
-    static constexpr int N = 2;
-    using type = float4;
-};
 
 // Shared-memory copy of the carry responses of a stage's operators, laid
 // out [operator][4][L] (see StageOp::resp), made once per CTA.

@@ -61,6 +61,8 @@ struct StageProgram {
     int aligned_only;   // refuse extents and addresses that need linesolve_any.cu
 };
 
+inline bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 // Number of (lines per CTA, chunk length, persistence, lines per thread)
 // configurations launch_stage knows in 0 .. 15; 16 is the one-thread-per-line
 // kernel (not a launch_stage configuration); 17, 18, 19 and 20 are
