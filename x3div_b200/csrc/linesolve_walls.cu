@@ -333,10 +333,11 @@ static int launch_wall_t(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, 
 // length out, o1 x o2 lines (the extents of the other two directions).
 // Four operators along y at 256 x 129 x 128 FP64 took 264 us on one thread per
 // line and take 92 us (2.9 TB/s of one read and one write each); fourteen at
-// 193^3 FP32 1634 and 345 us (2.3 TB/s).  What bounds them is L1 (about 70 %):
-// the five table rows, 16 bytes a load, beside the tile.  32 lines a CTA, where
-// every lane of a warp reads the same table entries, came to 361 us against 377
-// for 16, both before dependent launches.
+// 193^3 FP32 1634 and 345 us (2.3 TB/s).  What bounds them is latency at three
+// CTAs of 5 to 7 warps an SM (30 % of its warps) with L1 at 55 %: the five table
+// rows, 16 bytes a load, beside the tile.  32 lines a CTA, where every lane of a
+// warp reads the same table entries, came to 361 us against 377 for 16, both
+// before dependent launches.
 int launch_wall(x3d_ctx_s *ctx, const x3d_op_s *op, int kind, int dir, const void *in, void *out, int n_in, int o1,
                 int o2, int refl, bool fp32)
 {
